@@ -11,6 +11,10 @@ gbv_status set_error(gbv_status st, const char *msg);
 gbv_status check_launch(const char *what);
 gbv_status check_cuda(cudaError_t e, const char *what);
 
+// Stream-ordered scratch of a launch from the library's pool of the current
+// device (scratch.cpp); returned with cudaFreeAsync.
+cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
+
 // The device view of a parsed NanoVDB grid whose buffer is at d_grid
 // (nanovdb.cu).
 struct NvdbGrid;

@@ -1599,7 +1599,7 @@ inline gbv_status launch_render_t(const RenderParams &p, const Store &store, cud
   // bulk copy)
   int *pool = nullptr;
   const size_t maskBytes = (size_t)p.maskWords * 4;
-  st = check_cuda(cudaMallocAsync((void **)&pool, 256 + maskBytes, stream), "cudaMallocAsync(tile pool)");
+  st = check_cuda(scratch_alloc((void **)&pool, 256 + maskBytes, stream), "tile pool scratch");
   if (st != GBV_OK) return st;
   st = check_cuda(cudaMemsetAsync(pool, 0, sizeof(int), stream), "render_kernel: clearing the tile pool");
   RenderParams q = p;
