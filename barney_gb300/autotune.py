@@ -1,18 +1,17 @@
 """Autotuner for the batched persistent render launch.
 
 The batched launch has knobs that change its speed but never its images
-(every lane still renders its own pixels in the reference's accumulation
-order, and every brick shape stores the same cells; tests/test_gpu_batch.py
+(every pixel still accumulates in the reference's order, and every brick shape stores the same cells; tests/test_gpu_batch.py
 and tests/test_gpu_bricks.py check both bit for bit):
 
 * brick         -- log2 of the brick edge in cells per axis of the voxel
   stores (where neighbouring cells sit in HBM);
-* blocks_per_sm -- resident 288-thread blocks per SM (4, 5 or 6: the kernel
-  is compiled for each register budget);
-* threshold     -- a warp keeps traversing while at least this percentage of
-  its busy lanes still traces, then shades together;
-* skip          -- cell tests and distance draws a lane may make per traversal
-  iteration to reach its next sample position.
+* blocks_per_sm -- the register budget (4, 5 or 6 resident 128-thread blocks
+  per SM: the kernel is compiled for each);
+* threshold     -- a warp keeps tracing while at least this percentage of its
+  lanes does, or while no other stage has work for it;
+* skip          -- rounds (cell test, distance draw, step) a lane makes per
+  traversal iteration to reach its next sample position.
 
 tune_batch() times launch shapes of an existing batch; tuned_batch() also
 rebuilds the stores with each candidate brick shape (coordinate descent:
@@ -29,11 +28,11 @@ import json
 import os
 from pathlib import Path
 
-LAUNCH_CANDIDATES = [(b, t, k) for b in (4, 5, 6) for t in (5, 12, 20) for k in (4, 6, 8)]
+LAUNCH_CANDIDATES = [(b, t, k) for b in (4, 5, 6) for t in (15, 25, 40) for k in (4, 16, 64)]
 # What a launch shape means to the kernel (block size, traversal units); part
 # of every cache key, so choices cached by a build where the same numbers
 # meant another launch are not reused.
-LAUNCH_SHAPE_REVISION = "288-thread blocks, seek units"
+LAUNCH_SHAPE_REVISION = "block pool, seek rounds"
 BRICK_CANDIDATES = [(3, 3, 3), (2, 2, 2), (4, 4, 4), (4, 4, 2), (5, 3, 2)]
 
 

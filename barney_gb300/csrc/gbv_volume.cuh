@@ -192,20 +192,33 @@ struct XF {
   float lo, span, baseDensity;
 };
 
-__device__ __forceinline__ vec4 xf_map(const XF &xf, float s) {
-  float f = (s - xf.lo) / xf.span;
+// The two entries a value falls between and its weights.
+struct XFSegment {
+  float4 v0, v1;
+  float f, g;  // weight of v1, and 1 - f
+  __device__ __forceinline__ float opacity() const { return g * v0.w + f * v1.w; }
+  __device__ __forceinline__ vec3 color() const {
+    return vec3(g * v0.x + f * v1.x, g * v0.y + f * v1.y, g * v0.z + f * v1.z);
+  }
+};
+__device__ __forceinline__ XFSegment xf_segment(const XF &xf, float s) {
+  XFSegment r;
+  float f = s - xf.lo;
+  if (xf.span != 1.f) f /= xf.span;  // x / 1 is x: a domain of unit length needs no division
   f = clampv(f, 0.f, 1.f);
   f *= (float)(xf.n - 1);
-  int idx = clampv((int)f, 0, xf.n - 2);
+  const int idx = clampv((int)f, 0, xf.n - 2);
   f -= (float)idx;
-  const float4 v0 = __ldg(xf.v + idx), v1 = __ldg(xf.v + idx + 1);
-  vec4 r;
-  r.x = (1.f - f) * v0.x + f * v1.x;
-  r.y = (1.f - f) * v0.y + f * v1.y;
-  r.z = (1.f - f) * v0.z + f * v1.z;
-  r.w = (1.f - f) * v0.w + f * v1.w;
-  r.w *= xf.baseDensity;
+  r.v0 = __ldg(xf.v + idx);
+  r.v1 = __ldg(xf.v + idx + 1);
+  r.f = f;
+  r.g = 1.f - f;
   return r;
+}
+__device__ __forceinline__ vec4 xf_map(const XF &xf, float s) {
+  const XFSegment m = xf_segment(xf, s);
+  const vec3 c = m.color();
+  return vec4{c.x, c.y, c.z, m.opacity() * xf.baseDensity};
 }
 
 __host__ __device__ __forceinline__ float xf_majorant(const float4 *v, int n, float lo, float span, float bd,

@@ -255,6 +255,7 @@ static gbv_status render_frame(const char *fn, const gbv_scene *s, float *d_accu
   if (st != GBV_OK) return st;
   p.W = width;
   p.H = height;
+  p.aspect = (float)width / (float)height;
   p.accum = reinterpret_cast<float4 *>(d_accum);
   p.accumIdStart = accum_id_start;
   p.spp = spp;
@@ -398,6 +399,7 @@ extern "C" gbv_status gbv_render_noalloc(const gbv_scene *s, float *d_accum, int
   if (st != GBV_OK) return st;
   p.W = width;
   p.H = height;
+  p.aspect = (float)width / (float)height;
   p.accum = reinterpret_cast<float4 *>(d_accum);
   p.accumIdStart = accum_id_start;
   p.spp = spp;
@@ -428,7 +430,8 @@ extern "C" gbv_status gbv_batch_create(const gbv_scene *scenes, float *const *d_
     return set_error(GBV_ERROR_INVALID_ARGUMENT, "gbv_batch_create: bad argument");
   *out = nullptr;
   std::vector<RenderParams> items(count);
-  std::vector<long long> starts(count + 1, 0);
+  std::vector<long long> starts(count + 1, 0), outers(count + 1, 0);
+  int hits = 1;
   for (int i = 0; i < count; i++) {
     const gbv_scene *s = scenes + i;
     if (!s->d_voxels || !s->d_majorants || !s->d_tf || s->tf_n < 2 ||
@@ -449,32 +452,51 @@ extern "C" gbv_status gbv_batch_create(const gbv_scene *scenes, float *const *d_
     RenderParams &p = items[i];
     p.W = widths[i];
     p.H = heights[i];
+    p.aspect = (float)p.W / (float)p.H;
     p.accum = reinterpret_cast<float4 *>(d_accums[i]);
     p.maskWords = 0;
     p.cdfYOff = p.pivOff = p.rowOff = -1;
     p.pivPerRow = 0;
-    starts[i + 1] = starts[i] + (((long long)p.W + 7) / 8) * (((long long)p.H + 3) / 4);
+    const long long inner = plan_rect(p);
+    starts[i + 1] = starts[i] + inner;
+    outers[i + 1] = outers[i] + warp_tile_count(p) - inner;
+    const int h = path_hits(p);
+    if (h > hits) hits = h;
   }
-  if (starts[count] >= (1ll << 31) - (1ll << 20))
+  if (starts[count] + outers[count] >= (1ll << 31) - (1ll << 20))
     return set_error(GBV_ERROR_INVALID_ARGUMENT, "gbv_batch_create: more tiles than the 32-bit tile counter holds");
   gbv_batch *b = new gbv_batch();
   b->count = count;
   b->format = scenes[0].format;
   b->layout = scenes[0].layout;
-  b->totalTiles = starts[count];
+  b->innerTiles = starts[count];
+  b->outerTiles = outers[count];
+  starts.insert(starts.end(), outers.begin(), outers.end());
   b->occ = 4;
   b->threshold = kThresholdDefault;
-  b->skip = kSkipDefault;
+  b->skip = kBatchSkipDefault;
   gbv_status st = check_cuda(cudaGetDevice(&b->device), "gbv_batch_create: cudaGetDevice");
   if (st == GBV_OK) st = check_cuda(cudaMalloc((void **)&b->d_items, sizeof(RenderParams) * count), "gbv_batch_create");
   if (st == GBV_OK)
-    st = check_cuda(cudaMalloc((void **)&b->d_tileStart, sizeof(long long) * (count + 1)), "gbv_batch_create");
+    st = check_cuda(cudaMalloc((void **)&b->d_tileStart, sizeof(long long) * 2 * (count + 1)), "gbv_batch_create");
   if (st == GBV_OK) st = check_cuda(cudaMalloc((void **)&b->d_pool, sizeof(int)), "gbv_batch_create");
+  b->hits = hits;
+  if (st == GBV_OK) {
+    // the log of split tiles: room for kBatchLogPasses passes of every tile,
+    // at most kLogBytes (more passes split fewer tiles); without it none are
+    const size_t want = (size_t)b->innerTiles * 32 * log_words(hits) * sizeof(uint32_t) * kBatchLogPasses;
+    b->logBytes = want < kLogBytes ? want : kLogBytes;
+    if (cudaMalloc((void **)&b->d_log, b->logBytes) != cudaSuccess) {
+      cudaGetLastError();
+      b->d_log = nullptr;
+      b->logBytes = 0;
+    }
+  }
   if (st == GBV_OK)
     st = check_cuda(cudaMemcpy(b->d_items, items.data(), sizeof(RenderParams) * count, cudaMemcpyHostToDevice),
                     "gbv_batch_create: upload");
   if (st == GBV_OK)
-    st = check_cuda(cudaMemcpy(b->d_tileStart, starts.data(), sizeof(long long) * (count + 1),
+    st = check_cuda(cudaMemcpy(b->d_tileStart, starts.data(), sizeof(long long) * 2 * (count + 1),
                                cudaMemcpyHostToDevice),
                     "gbv_batch_create: upload");
   if (st != GBV_OK) {
@@ -525,6 +547,7 @@ extern "C" gbv_status gbv_batch_destroy(gbv_batch *b) {
   if (b->d_items) cudaFree(b->d_items);
   if (b->d_tileStart) cudaFree(b->d_tileStart);
   if (b->d_pool) cudaFree(b->d_pool);
+  if (b->d_log) cudaFree(b->d_log);
   delete b;
   return GBV_OK;
 }

@@ -2,13 +2,14 @@
 // code, the persistent kernel and its launch templates (instantiated once per
 // voxel store in render_store_*.cu).
 //
-// One thread owns one pixel for all of a launch's accumulation passes, so
-// the frame buffer needs no atomics and every pixel accumulates its
-// fragments in the reference's order (pass-major, then generation; within a
-// generation the shadow ray before the bounce ray).  A pass follows
-// Context::renderTiles (barney/Context.cpp:142-185): _generateRays, then per
-// generation the trace (MCVolumeAccel::isProg) and _shadeRays/bounce
-// (barney/kernels/shadeRays.cu:477-1041) of the pixel's queued rays.
+// Every pixel accumulates its fragments in the reference's order (pass-major,
+// then generation; within a generation the shadow ray before the bounce ray)
+// with plain adds: a path sums its pixel's passes one after the other, or
+// logs one pass's fragments, which a second kernel adds up in that order.  A
+// pass follows Context::renderTiles (barney/Context.cpp:142-185):
+// _generateRays, then per generation the trace (MCVolumeAccel::isProg) and
+// _shadeRays/bounce (barney/kernels/shadeRays.cu:477-1041) of the pixel's
+// queued rays.
 #pragma once
 #include <cstring>
 #include <mutex>
@@ -39,6 +40,7 @@ struct RenderParams {
   // camera (PerspectiveCamera::commit)
   vec3 lens00, dir00, du, dv;
   int W, H;
+  float aspect;  // W / H
   int numDir;
   DirLightDev dir[4];
   int hasEnv;
@@ -51,8 +53,8 @@ struct RenderParams {
   int accumIdStart, spp;
   unsigned long long *counters;
   int *capFlag;   // if set, a loop-cap event stores 1 here (no counting needed)
-  int skip;       // empty macrocells crossed per traversal step
-  int threshold;  // keep traversing while at least this % of busy lanes trace
+  int skip;       // seek rounds per traversal iteration
+  int threshold;  // keep tracing while at least this % of the lanes does
   // shared-memory staging (offsets in 32-bit words of the dynamic smem)
   int maskWords;  // >0: bitmask of non-zero majorants staged at offset 0 (a multiple of 4 words)
   const uint32_t *maskSrc;  // the bitmask in HBM (16-byte aligned), staged by one bulk copy; null: by ballots
@@ -61,6 +63,17 @@ struct RenderParams {
   int pivPerRow;
   int rowOff;     // >=0: per env-map row (pdf_y, pdf denominator) staged here
   int profile;    // accumulate per-phase cycle counts
+  int poolOff;    // the block's path pool starts here
+  int slots;      // path slots a block uses (a multiple of 32)
+  // The warp tiles that may see the field (its projection's rectangle, in
+  // tiles): handed out first, numbered row by row; the other tiles follow
+  int rx, ry, rw, rh;
+  // What the launch hands out: `whole` inner tiles with all their passes, then
+  // each pass of `split` inner tiles by itself (its fragments logged and added
+  // up in order by resolve_kernel), then the outer tiles
+  long long whole, split, outer;
+  uint32_t *log;  // null: split == 0
+  int logHits;    // fragments a record has room for
   int maskMode;   // 0: the staged bitmask arrives by one bulk copy of a precomputed mask; 1: by ballots
   // voxel store of this scene (see make_store)
   const void *vox;
@@ -101,6 +114,46 @@ __host__ __device__ inline long long owned_ref_tiles(int W, int H, int rank, int
 __host__ __device__ inline long long warp_tile_count(const RenderParams &p) {
   if (p.numRanks > 1) return owned_ref_tiles(p.W, p.H, p.rank, p.numRanks) * 32;
   return (((long long)p.W + 7) >> 3) * (((long long)p.H + 3) >> 2);
+}
+
+// what one launch hands out (see RenderParams::whole)
+__host__ __device__ inline long long launch_tiles(const RenderParams &L) { return L.whole + L.split * L.spp + L.outer; }
+// the i-th tile inside (outside) the field's rectangle, row-major
+__device__ __forceinline__ int inner_tile(const RenderParams &p, int i) {
+  const int tilesX = (int)(((long long)p.W + 7) >> 3);
+  return p.rw == 0 ? i : (p.ry + i / p.rw) * tilesX + p.rx + i % p.rw;
+}
+__device__ __forceinline__ int outer_tile(const RenderParams &p, int i) {
+  const int tilesX = (int)(((long long)p.W + 7) >> 3), side = tilesX - p.rw;
+  if (i < p.ry * tilesX) return i;  // the rows before the rectangle
+  i -= p.ry * tilesX;
+  if (i >= p.rh * side) return (p.ry + p.rh) * tilesX + i - p.rh * side;  // the rows after it
+  const int col = i % side;
+  return (p.ry + i / side) * tilesX + (col < p.rx ? col : col + p.rw);
+}
+// the last item whose first tile is at or before t
+__device__ __forceinline__ int tile_item(const long long *__restrict__ start, int numItems, long long t) {
+  int lo = 0, hi = numItems - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (start[mid] <= t) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+// a warp tile's upper-left pixel
+template <bool Batch>
+__device__ __forceinline__ void tile_corner(const RenderParams &L, const RenderParams &tp, int tile, int &tx, int &ty) {
+  if (!Batch && L.numRanks > 1) {  // the k-th 32x32 tile this rank owns, 4x8 warp tiles in it
+    const long long big = (long long)L.rank + (long long)(tile >> 5) * L.numRanks;
+    const int bigX = (int)(((long long)tp.W + kRefTile - 1) / kRefTile);
+    tx = (int)(big % bigX) * kRefTile + (tile & 3) * 8;
+    ty = (int)(big / bigX) * kRefTile + ((tile >> 2) & 7) * 4;
+  } else {
+    const int tilesX = (int)(((long long)tp.W + 7) >> 3);
+    tx = (tile % tilesX) * 8;
+    ty = (tile / tilesX) * 4;
+  }
 }
 
 template <class Store> __device__ __forceinline__ Store make_store(const RenderParams &p);
@@ -675,16 +728,6 @@ __device__ __forceinline__ void bounce_volume_hit(const RenderParams &p, PathRay
   }
 }
 
-// Out-of-line copies of the shading helpers for the batched kernel: its
-// lanes read their scenes' parameters from global memory (one record per
-// item), and inlined helpers keep more of them live than the registers hold
-// (measured on the 64-item workload: 13% slower inlined).  The one-scene
-// kernel inlines the helpers themselves.
-static __device__ __noinline__ void bounce_volume_hit_ool(const RenderParams &p, PathRay &ray, const Hit &h, vec3 P,
-                                                      int pathDepth, Random &random, const EnvPick &pick,
-                                                      ShadeOut &out) {
-  bounce_volume_hit(p, ray, h, P, pathDepth, random, pick, out);
-}
 // owl::common::frame: the orthonormal frame about a unit normal N that
 // xfmVector(frame(N), v) uses -- dx the longer of (1,0,0) x N and
 // (0,1,0) x N, normalized, dy = normalize(N x dx)
@@ -784,14 +827,6 @@ static __device__ __noinline__ void bounce_surface_hit(const RenderParams &p, Pa
   }
 }
 
-static __device__ __noinline__ float4 tex2D_ool(const EnvDev &e, float u, float v) { return tex2D(e, u, v); }
-static __device__ __noinline__ float2 env_miss_coords_ool(const RenderParams &p, vec3 rayDir) {
-  return env_miss_coords(p, rayDir);
-}
-static __device__ __noinline__ EnvPick env_pick_coords_ool(const RenderParams &p, Random &r) {
-  return env_pick_coords(p, r);
-}
-
 __device__ __forceinline__ void accum_add(float4 &acc, vec3 frag) {
   if (frag.x > 0.f) acc.x += frag.x;
   if (frag.y > 0.f) acc.y += frag.y;
@@ -807,12 +842,27 @@ __device__ __forceinline__ void accum_add(float4 &acc, vec3 frag) {
 // kSkipDefault) cell tests and distance draws to reach its next sample
 // position, then the warp's ready lanes take their density samples together.
 // -------------------------------------------------------------------------
-// Defaults of the launch shape (the best of a same-box sweep of 3..64 units
-// per seek and thresholds 3..30% on the 512^3 1080p frame; units 5..8 with
-// thresholds 16..25 are within 1% of each other; results never depend on
-// them)
-constexpr int kSkipDefault = 6;
-constexpr int kThresholdDefault = 20;
+// Defaults of the launch shape and the scheduling limits of the frame kernel
+// (512^3 1080p 16-pass frame / 256^3 720p 1 pass; results never depend on
+// them):
+// * rounds a seek makes before the warp samples: 2: 12.3 / 0.507 ms, 3:
+//   12.1 / 0.498, 4: 11.7 / 0.502;
+// * a warp leaves tracing for a waiting stage below this share of its lanes:
+//   10%: 12.8 / 0.69, 20%: 12.0 / 0.69, 30%: 11.5 / 0.71, 50%: 11.9 / 0.73,
+//   65%: slower by 10% or more on the small frames;
+// * kRefillMin, the rays a refill waits for: 4: 12.0 / 0.70, 8: 11.8 / 0.69,
+//   12: 11.7 / 0.67;
+// * kFull, the paths that make a stage worth leaving another for: 16: 11.9 /
+//   0.71, 24: 11.8 / 0.69, 30: 11.7 / 0.69.
+constexpr int kSkipDefault = 4;
+// A batch's lanes read their scene's record from memory at every seek: one
+// that goes on to its next position reads it less often (64 uneven scenes, 8
+// passes: 4 rounds 6.25 ms, 16: 5.83, 64: 5.53).
+constexpr int kBatchSkipDefault = 64;
+constexpr int kThresholdDefault = 25;
+constexpr int kRefillMin = 12, kFull = 28;
+constexpr int kRepeatMin = 24;     // lanes for which starting passes goes on
+constexpr int kIdlePolls = 4096;   // polls (200 ns) of a warp without work
 
 // Per-lane event counts; with On == false the counting and its registers
 // compile away (timed launches pass no counter buffer).
@@ -834,7 +884,6 @@ struct Traversal {
   int cx, cy, cz;
   int stopx, stopy, stopz;
   float ray_t0, tMax, ncb;
-  float tc;            // t_closest of the current cell
   float t, segHi, maj; // delta tracking in the current cell
   Random rng;
   int inCell;
@@ -912,85 +961,78 @@ __device__ __forceinline__ bool trace_begin(const FieldGeom &F, const MCGridDev 
   return true;
 }
 
-// next_cell_begin = t_closest, then step every axis whose t_next equals it
-__device__ __forceinline__ bool trace_advance(Traversal &T, float tc, bool sx, bool sy, bool sz) {
+// next_cell_begin = t_closest, then step every axis whose t_next equals it;
+// false when the ray leaves the grid (its state is then not used again).
+// Selects instead of branches: every lane that steps runs the same code.
+__device__ __forceinline__ bool trace_advance(Traversal &T, float tc) {
+  const bool ax = T.t_next.x == tc, ay = T.t_next.y == tc, az = T.t_next.z == tc;
   T.ncb = tc;
-  if (T.t_next.x == tc) {
-    T.t_next.x += T.t_step.x;
-    T.cx += sx ? 1 : -1;
-    if (T.cx == T.stopx) return false;
-  }
-  if (T.t_next.y == tc) {
-    T.t_next.y += T.t_step.y;
-    T.cy += sy ? 1 : -1;
-    if (T.cy == T.stopy) return false;
-  }
-  if (T.t_next.z == tc) {
-    T.t_next.z += T.t_step.z;
-    T.cz += sz ? 1 : -1;
-    if (T.cz == T.stopz) return false;
-  }
-  return true;
+  T.t_next.x = ax ? T.t_next.x + T.t_step.x : T.t_next.x;
+  T.t_next.y = ay ? T.t_next.y + T.t_step.y : T.t_next.y;
+  T.t_next.z = az ? T.t_next.z + T.t_step.z : T.t_next.z;
+  T.cx += ax ? (T.stopx >> 31) | 1 : 0;
+  T.cy += ay ? (T.stopy >> 31) | 1 : 0;
+  T.cz += az ? (T.stopz >> 31) | 1 : 0;
+  return !((T.cx == T.stopx) | (T.cy == T.stopy) | (T.cz == T.stopz));
 }
 
 // The traversal is split so that the expensive part, the density sample,
 // runs for all of a warp's tracing lanes at once.  trace_seek advances a lane
-// to its next sample position: it crosses empty macrocells, enters the next
-// cell of non-zero majorant and draws Woodcock distances until one falls
-// inside the current cell (T.inCell = 2: a position is ready), at most
-// `units` cell tests and distance draws per call.  trace_sample then
-// samples there and makes the accept test.  Every lane performs exactly the
-// operations, in exactly the order, of the one-step-at-a-time loop
-// (dda::dda3 with Woodcock::sampleRange inside each cell); only the grouping
-// of a lane's steps into warp iterations differs.
+// toward its next sample position (T.inCell = 2: a position is ready) by at
+// most `rounds` rounds of: test the macrocell it stands before (T.inCell 0;
+// 1: inside one of non-zero majorant), draw a Woodcock distance inside it,
+// and, from an empty cell or past the cell's end, step to the next cell.
+// trace_sample then samples there and makes the accept test.  Every lane
+// performs exactly the operations, in exactly the order, of the
+// one-step-at-a-time loop (dda::dda3 with Woodcock::sampleRange inside each
+// cell); only the grouping of a lane's steps into warp iterations differs.
+// A round has one copy of each step and the lanes meet again after each, so
+// that lanes crossing empty cells and lanes leaving a cell step together.
 template <class Cnt>
-__device__ __forceinline__ int trace_seek(const MCGridDev &G, Traversal &T, Cnt &cnt, int units, bool staged,
+__device__ __forceinline__ int trace_seek(const MCGridDev &G, Traversal &T, Cnt &cnt, int rounds, bool staged,
                                           int *capFlag) {
-  const bool sx = T.stopx >= 0, sy = T.stopy >= 0, sz = T.stopz >= 0;
   const int maxCells = G.M[0] + G.M[1] + G.M[2] + 8;
-  for (int k = 0; k < units; k++) {
-    if (!T.inCell) {
+  int state = TR_CONTINUE;
+#pragma unroll 1
+  for (int round = 0; round < rounds && T.inCell != 2 && state == TR_CONTINUE; round++) {
+    const float tc = reduce_min(T.t_next);
+    bool step = false;
+    if (T.inCell == 0) {
       GBV_COUNT(cnt, cells);
+      const int ci = T.cx + G.M[0] * (T.cy + G.M[1] * T.cz);
+      const bool nonzero = staged ? ((g_smem[ci >> 5] >> (ci & 31)) & 1u) != 0u : __ldg(G.maj + ci) != 0.f;
       if (++T.cells > maxCells) {
         GBV_COUNT(cnt, caps);
         if (capFlag) *capFlag = 1;
-        return TR_MISS;
+        state = TR_MISS;
+      } else if (nonzero) {
+        T.maj = __ldg(G.maj + ci);
+        T.inCell = 1;
+        T.t = T.ray_t0 + T.ncb;
+        T.segHi = mn(T.ray_t0 + mn(tc, T.tMax), T.rayTMax);
+        T.steps = 0;
+        GBV_COUNT(cnt, mcs);
+      } else {
+        step = true;
       }
-      const float tc = reduce_min(T.t_next);
-      const int ci = T.cx + G.M[0] * (T.cy + G.M[1] * T.cz);
-      const bool nonzero = staged ? ((g_smem[ci >> 5] >> (ci & 31)) & 1u) != 0u : __ldg(G.maj + ci) != 0.f;
-      if (!nonzero) {
-        if (!trace_advance(T, tc, sx, sy, sz)) return TR_MISS;
-        continue;
-      }
-      const float maj = __ldg(G.maj + ci);
-      const float cell_t0 = T.ray_t0 + T.ncb;
-      const float cell_t1 = T.ray_t0 + mn(tc, T.tMax);
-      T.inCell = 1;
-      T.tc = tc;
-      T.maj = maj;
-      T.t = cell_t0;
-      T.segHi = mn(cell_t1, T.rayTMax);
-      T.steps = 0;
-      GBV_COUNT(cnt, mcs);
     }
-    // one Woodcock distance
-    const float r = T.rng();
-    const float dt = -fastLog(1.f - r) / T.maj;
-    T.t += dt;
-    if (T.t >= T.segHi || ++T.steps > kWoodcockCap) {
-      if (T.steps > kWoodcockCap) {
-        GBV_COUNT(cnt, caps);
-        if (capFlag) *capFlag = 1;
+    if (T.inCell == 1) {
+      const float r = T.rng();
+      const float dt = -fastLog(1.f - r) / T.maj;
+      T.t += dt;
+      T.inCell = 2;
+      if (T.t >= T.segHi || ++T.steps > kWoodcockCap) {
+        if (T.steps > kWoodcockCap) {
+          GBV_COUNT(cnt, caps);
+          if (capFlag) *capFlag = 1;
+        }
+        T.inCell = 0;
+        step = true;
       }
-      T.inCell = 0;
-      if (!trace_advance(T, T.tc, sx, sy, sz)) return TR_MISS;
-      continue;
     }
-    T.inCell = 2;
-    return TR_CONTINUE;
+    if (step && !trace_advance(T, tc)) state = TR_MISS;
   }
-  return TR_CONTINUE;
+  return state;
 }
 
 template <class Store, class Cnt>
@@ -998,12 +1040,19 @@ __device__ __forceinline__ int trace_sample(const FieldGeom &F, const Store &sto
                                             Hit &h, Cnt &cnt) {
   T.inCell = 1;
   const vec3 P = T.org + T.t * T.dir;
-  const vec4 smp = sample_and_map(F, store, xf, P);
+  // Volume::DD::sampleAndMap (Volume.h:66-80): NaN maps to zeros
+  const float f = sample_field(F, store, P);
   GBV_COUNT(cnt, samples);
-  if (smp.w >= T.rng() * T.maj) {
+  float w = 0.f;
+  XFSegment seg;
+  if (!isnan(f)) {
+    seg = xf_segment(xf, f);
+    w = seg.opacity() * xf.baseDensity;
+  }
+  if (w >= T.rng() * T.maj) {
     h.hit = true;
     h.t = T.t;
-    h.rgb = vec3(smp.x, smp.y, smp.z);
+    h.rgb = isnan(f) ? vec3(0.f) : seg.color();
     return TR_HIT;
   }
   return TR_CONTINUE;
@@ -1027,7 +1076,6 @@ __device__ __forceinline__ bool iso_search(const FieldGeom &F, const Store &rend
                                            float stop = __int_as_float_hd(0x7f800000)) {
   // the sub-steps' samples lie close together along the ray: read through L1
   const auto &store = via_l1(renderStore);
-  const bool sx = T.stopx >= 0, sy = T.stopy >= 0, sz = T.stopz >= 0;
   const int maxCells = G.M[0] + G.M[1] + G.M[2] + 8;
   float tHit = tmax;
   bool stopped = false;
@@ -1062,7 +1110,7 @@ __device__ __forceinline__ bool iso_search(const FieldGeom &F, const Store &rend
         }
       }
     }
-    if (stopped || !trace_advance(T, tc, sx, sy, sz)) break;
+    if (stopped || !trace_advance(T, tc)) break;
   }
   if (!(tHit < tmax)) return false;
   const vec3 P = T.org + tHit * T.dir;
@@ -1178,24 +1226,41 @@ static __device__ __noinline__ void write_aux(const RenderParams &p, size_t px, 
 }
 
 // -------------------------------------------------------------------------
-// The persistent frame kernel.  Each lane owns one pixel for all of the
-// launch's passes, so fragments accumulate in the reference's order
-// (pass-major, generation, shadow ray before bounce ray) without atomics.
-// Warps take 8x4-pixel tiles from a global pool; a lane whose pixel is done
-// takes the next pixel of its warp's tile.  Every loop iteration advances a
-// lane by one bounded unit: a trace step, or a shade and the set-up of the
-// next trace.
+// The persistent frame kernel.  A path lives in a slot of its block's pool in
+// shared memory; a block (one per SM) has more paths than lanes.  A warp takes
+// up to 32 paths that wait for the same stage and runs that stage for them:
+// starting passes and shading misses, tracing, the iso-surface search, shading
+// hits.
+//
+// What bounds it: instruction issue.  A ray is a few cells, draws and samples
+// of very different number, a hit's shading a few thousand instructions; a
+// lane that owns its pixel from generation to shading leaves the others of
+// its warp waiting in every phase (8.6 of 32 lanes active per instruction),
+// and warps in different phases evict one another's code (41% of the stall
+// cycles were instruction fetch).  Taking paths by stage gives 15 to 20 active
+// lanes; letting the block's warps leave tracing for shading together
+// (PathPool::shading) keeps them in the same code: 16.2 -> 14.5 ms from the
+// pool, -> 12.4 ms from the common phase, -> 11.7 ms from refilling lanes in
+// batches (512^3, 1080p, 16 passes).  128 registers a thread (16 warps) with
+// next to no spills beat 24 warps of 80 registers (12.9 ms).
+//
+// A path that sums all of its pixel's passes runs them one after the other,
+// so the last pixels' passes hold a small frame's end: 50 to 80% of its time.
+// The tiles that see the field come first and, as far as the log has room,
+// pass by pass (F_SPLIT), each pass's fragments logged: 256^2 x 16 passes of a
+// 64^3 volume 0.65 -> 0.18 ms, 853x479 x 8 passes 1.27 -> 0.38 ms, 1280x720 x
+// 4 passes multi-scatter 2.83 -> 1.24 ms.
 // -------------------------------------------------------------------------
-// 9 warps per block: at 4 resident blocks per SM (36 warps) the register
-// budget is 56 per thread (measured fastest: 256 x 5 with 48 registers
-// -4.2%, 192 x 6 -2%)
-constexpr int kThreads = 288;
-enum { K_NONE = 0, K_MAIN = 1, K_SHADOW = 2 };
+// Path slots of a block
+constexpr int kSlots = 1024;
+// Threads of a block, by the register budget gbv_render_config.blocks_per_sm
+// asks for (4: 128 registers a thread, 5: 96, 6: 80)
+__host__ __device__ constexpr int block_threads(int budget) { return budget * 128; }
 
 __device__ __forceinline__ float4 miss_color(const RenderParams &p, int iy) {
-  const float t = ((float)iy + .5f) / (float)p.H;
   float4 m = p.bg;
   if (!(p.bg.w >= 0.f)) {
+    const float t = ((float)iy + .5f) / (float)p.H;
     m.x = (1.0f - t) * 0.9f + t * 0.15f;
     m.y = (1.0f - t) * 0.9f + t * 0.25f;
     m.z = (1.0f - t) * 0.9f + t * .8f;
@@ -1206,14 +1271,13 @@ __device__ __forceinline__ float4 miss_color(const RenderParams &p, int iy) {
 
 // _generateRays (generateRays.cu:72-243), perspective camera, no aperture
 __device__ __forceinline__ void generate_primary(const RenderParams &p, int ix, int iy, int accumID, PathRay &ray) {
-  const float aspect = (float)p.W / (float)p.H;
   Random rand = Random::from_pair((unsigned)(ix + p.W * accumID), (unsigned)(iy + p.H * accumID));
   ray.seed = seeded((uint32_t)(ix + accumID * p.W), (uint32_t)iy);
   const float pixel_u = (accumID == 0) ? .5f : rand();
   const float pixel_v = (accumID == 0) ? .5f : rand();
   const float image_u = ((float)ix + pixel_u) / (float)p.W;
   const float image_v = ((float)iy + pixel_v) / (float)p.H;
-  const vec3 d = p.dir00 + (1.f * aspect * (image_u - .5f)) * p.du + (1.f * (image_v - .5f)) * p.dv;
+  const vec3 d = p.dir00 + (1.f * p.aspect * (image_u - .5f)) * p.du + (1.f * (image_v - .5f)) * p.dv;
   ray.org = p.lens00;
   ray.dir = normalize(d);
   ray.tMax = 1e30f;
@@ -1223,28 +1287,196 @@ __device__ __forceinline__ void generate_primary(const RenderParams &p, int ix, 
   ray.numDiffuseBounces = 0;
 }
 
+// What a path waits for; each is a bitmask over the block's slots in shared
+// memory.  Publishing a path sets its bit (after a fence), taking it clears
+// the bit: whoever clears it owns the path.
+enum {
+  Q_FREE = 0,   // no pixel
+  Q_START = 1,  // F_FRESH: its next pass is to be generated; else its main ray left the world
+  Q_READY = 2,  // a ray (F_SHADOW: the shadow ray) is to be traced
+  Q_HIT = 3,    // its main ray has a hit to shade
+  Q_ISO = 4,    // the volume is traced, the iso-surface search is to run
+  Q_COUNT = 5
+};
+// Control word of a path: flags, generation in bits 8..15
+constexpr uint32_t F_FRESH = 1u, F_SHADOW = 2u, F_ALIVE = 4u, F_ISOBOX = 8u, F_SPLIT = 16u,
+                   F_LONE = 32u /* a shadow ray of a path that goes on elsewhere */,
+                   F_OUTER = 64u /* a pixel outside the field's rectangle */, F_VOLHIT = 1u << 16, F_SURFHIT = 2u << 16,
+                   kHitMask = 3u << 16;
+// Words of a path's record.  The main ray's hit (t, rgb, the surface's
+// normal) shares the shadow ray's words: a main ray's hit is shaded before
+// its shadow ray exists.
+// A split path (one pass of a pixel, F_SPLIT) keeps no sum: W_ACC holds its
+// record's index in the log and the fragments it has logged.
+enum {
+  W_REC = 23, W_MASK = 24,
+  W_ORG = 0, W_DIR = 3, W_SEED = 6, W_TP = 8 /* 3 halves, bounce counts */, W_MIS = 10,
+  W_SORG = 11, W_SDIR = 14, W_STMAX = 17, W_SSEED = 18, W_STP = 20, W_SMIS = 22,
+  W_HT = 11, W_HRGB = 12, W_HN = 15,
+  W_ACC = 23, W_IX = 27, W_IY = 28, W_PASS = 29, W_CTL = 30, W_ITEM = 31, W_ISORNG = 32
+};
+
+// Record of a split path in the log: the fragments it logged (a bit per
+// generation; kLogMissed: the primary ray itself missed), the pass's alpha,
+// then 3 floats per generation -- the shadow ray's fragment of a hit, or the
+// miss that ends the path.  Each generation adds at most one fragment to a
+// pixel that is not zero, so adding a pixel's records pass by pass and
+// generation by generation is the order in which a lane that owned the pixel
+// would add them.
+constexpr uint32_t kLogMissed = 1u << 31;
+__host__ __device__ constexpr int log_words(int hits) { return 2 + 3 * hits; }
+__device__ __forceinline__ void log_fragment(const RenderParams &L, uint32_t rec, int gen, vec3 f) {
+  if (gen >= L.logHits) return;  // path_hits bounds the generations
+  float *r = reinterpret_cast<float *>(L.log) + (size_t)rec * log_words(L.logHits) + 2 + 3 * gen;
+  r[0] = f.x;
+  r[1] = f.y;
+  r[2] = f.z;
+}
+__device__ __forceinline__ void log_end(const RenderParams &L, uint32_t rec, uint32_t mask, float alpha) {
+  uint32_t *r = L.log + (size_t)rec * log_words(L.logHits);
+  r[0] = mask;
+  r[1] = __float_as_uint(alpha);
+}
+
+// Position of the r-th set bit (r < popc(bits)).
+__device__ __forceinline__ int nth_bit(uint32_t bits, int r) {
+  int p = 0;
+#pragma unroll
+  for (int h = 16; h > 0; h >>= 1) {
+    const int t = __popc(bits & ((1u << h) - 1u));
+    const bool up = r >= t;
+    r -= up ? t : 0;
+    p += up ? h : 0;
+    bits = up ? bits >> h : bits;
+  }
+  return p;
+}
+__device__ __forceinline__ int warp_scan(int v) {  // inclusive sum over the warp's lanes
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, v, o);
+    if ((int)(threadIdx.x & 31) >= o) v += x;
+  }
+  return v;
+}
+
+// The paths of one block, field-major: lane k of a stage reads word f of
+// slot j at bank j mod 32.
+template <bool Iso> struct PathPool {
+  static constexpr int kWords = Iso ? 34 : 32;
+  static constexpr int kStride = kWords * kSlots + Q_COUNT * (kSlots / 32) + 1 + 6 * 24;
+  uint32_t *w;
+  __device__ __forceinline__ uint32_t u(int f, int k) const { return w[f * kSlots + k]; }
+  __device__ __forceinline__ void setu(int f, int k, uint32_t v) const { w[f * kSlots + k] = v; }
+  __device__ __forceinline__ float f(int i, int k) const { return __uint_as_float(w[i * kSlots + k]); }
+  __device__ __forceinline__ void setf(int i, int k, float v) const { w[i * kSlots + k] = __float_as_uint(v); }
+  __device__ __forceinline__ vec3 v3(int i, int k) const { return vec3(f(i, k), f(i + 1, k), f(i + 2, k)); }
+  __device__ __forceinline__ void setv3(int i, int k, vec3 v) const {
+    setf(i, k, v.x);
+    setf(i + 1, k, v.y);
+    setf(i + 2, k, v.z);
+  }
+  __device__ __forceinline__ uint64_t u64(int i, int k) const {
+    return (uint64_t)u(i, k) | ((uint64_t)u(i + 1, k) << 32);
+  }
+  __device__ __forceinline__ void setu64(int i, int k, uint64_t v) const {
+    setu(i, k, (uint32_t)v);
+    setu(i + 1, k, (uint32_t)(v >> 32));
+  }
+  __device__ __forceinline__ float4 acc(int k) const {
+    return make_float4(f(W_ACC, k), f(W_ACC + 1, k), f(W_ACC + 2, k), f(W_ACC + 3, k));
+  }
+  __device__ __forceinline__ void setacc(int k, float4 a) const {
+    setf(W_ACC, k, a.x);
+    setf(W_ACC + 1, k, a.y);
+    setf(W_ACC + 2, k, a.z);
+    setf(W_ACC + 3, k, a.w);
+  }
+  __device__ __forceinline__ vec3h half3(int i, int k) const {
+    const uint32_t a = u(i, k), b = u(i + 1, k);
+    return vec3h{(uint16_t)(a & 0xffffu), (uint16_t)(a >> 16), (uint16_t)(b & 0xffffu)};
+  }
+  __device__ __forceinline__ void sethalf3(int i, int k, vec3h h, uint32_t upper = 0) const {
+    setu(i, k, (uint32_t)h.x | ((uint32_t)h.y << 16));
+    setu(i + 1, k, (uint32_t)h.z | (upper << 16));
+  }
+  __device__ __forceinline__ uint32_t *queue(int q) const { return w + kWords * kSlots + q * (kSlots / 32); }
+  // Hands path k to whoever takes it from queue q.
+  __device__ __forceinline__ void publish(int q, int k) const {
+    __threadfence_block();
+    atomicOr(queue(q) + (k >> 5), 1u << (k & 31));
+  }
+  // The block's phase: whether warps leave tracing for the shading stages
+  // (whole warp; one lane's read, so that the warp agrees).
+  __device__ __forceinline__ bool shading() const {
+    const volatile uint32_t *m = queue(Q_COUNT);
+    return __shfl_sync(0xffffffffu, *m, 0) != 0u;
+  }
+  __device__ __forceinline__ void set_shading(uint32_t on) const {
+    volatile uint32_t *m = queue(Q_COUNT);
+    if ((threadIdx.x & 31) == 0) *m = on;
+    __syncwarp();
+  }
+  // Paths waiting in queue q (whole warp).
+  __device__ __forceinline__ int waiting(int q) const {
+    const volatile uint32_t *m = queue(q);
+    return (int)__reduce_add_sync(0xffffffffu, (unsigned)__popc(m[threadIdx.x & 31]));
+  }
+  // Takes up to `want` (<= 32) paths from queue q (whole warp): lane i gets
+  // the i-th of the n taken, other lanes -1.  rot spreads the warps over the
+  // queue's words.
+  __device__ __forceinline__ int take(int q, int want, int rot, int &n) const {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    volatile uint32_t *m = queue(q);
+    const int at = (lane + rot) & 31;
+    const uint32_t bits = m[at];
+    const int c = __popc(bits);
+    const int before = warp_scan(c) - c;
+    const int mine = min(max(want - before, 0), c);
+    const uint32_t sel = mine == c ? bits : bits & ((1u << nth_bit(bits, mine)) - 1u);
+    const uint32_t got = sel ? atomicAnd(const_cast<uint32_t *>(m) + at, ~sel) & sel : 0u;
+    __threadfence_block();
+    const int g = __popc(got), upTo = warp_scan(g);
+    n = __shfl_sync(FULL, upTo, 31);
+    const int first = upTo - g;
+    int l = 0;  // the word lane i's path is in: the last one that starts at or before i
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) {
+      const int x = __shfl_sync(FULL, first, l + h);
+      l += x <= lane ? h : 0;
+    }
+    const uint32_t word = __shfl_sync(FULL, got, l);
+    const int r = lane - __shfl_sync(FULL, first, l);
+    return lane < n ? ((l + rot) & 31) * 32 + nth_bit(word, r) : -1;
+  }
+};
+
 // Batch: the launch renders `numItems` scenes (items[]), whose 8x4-pixel
 // tiles are numbered consecutively (tileStart[] holds the prefix sums); a
-// lane reads the scene of the pixel it owns.  Otherwise the launch renders
+// lane reads the scene of the path it works on.  Otherwise the launch renders
 // the one scene `p0`.  Launch-wide settings (passes, thresholds, counters)
 // always come from p0.  Count: whether to count events (see Ctr) and, with
 // a profile requested in the launch config (gbv_render_config.profile),
 // cycles and lanes per phase (the timed kernel, Count =
 // false, carries no profiling code).
-// p0 is __grid_constant__ so that helpers (inlined, or the batched kernel's
-// out-of-line copies) can take it by reference without a copy to local
-// memory.
+// p0 is __grid_constant__ so that helpers can take it by reference without a
+// copy to local memory.
 // Iso: the world holds an iso-surface (p0.isoOn; never batched): each trace
 // also runs its intersection program, before the volume's when its instance
 // index is the lower one (p0.isoFirst) and otherwise after it, each bounded
 // by the other's hit, and shading takes the surface branch on its hits.
-template <class Store, int MinBlocks, bool Batch, bool Count, bool Iso = false>
-__global__ void __launch_bounds__(kThreads, MinBlocks)
+template <class Store, int Budget, bool Batch, bool Count, bool Iso = false>
+__global__ void __launch_bounds__(block_threads(Budget), 1)
     render_kernel(const __grid_constant__ RenderParams p0, const RenderParams *__restrict__ items,
                   const long long *__restrict__ tileStart, int numItems, int *__restrict__ pool) {
   static_assert(!(Iso && Batch), "batched launches render volume-only worlds");
+  using Pool = PathPool<Iso>;
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
+  const float INF = __int_as_float(0x7f800000);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const int rot = 2 * warp;
   const RenderParams &L = p0;  // launch-wide settings
   // ---- stage the majorant bitmask and env-map tables in shared memory ----
   if (!Batch) {
@@ -1263,269 +1495,528 @@ __global__ void __launch_bounds__(kThreads, MinBlocks)
     if (p.rowOff >= 0)
       for (int i = threadIdx.x; i < p.env.H; i += blockDim.x)
         reinterpret_cast<float2 *>(g_smem + p.rowOff)[i] = env_row_terms(p.env, i);
-    __syncthreads();
   }
-  const long long numTiles = Batch ? tileStart[numItems] : warp_tile_count(p0);
+  const Pool P{g_smem + L.poolOff};
+  for (int i = threadIdx.x; i <= Q_COUNT * (kSlots / 32); i += blockDim.x)
+    P.queue(0)[i] = i < L.slots / 32 ? 0xffffffffu : 0u;  // slots [0, L.slots) are free
+  __syncthreads();
+  if (lane == 0) P.queue(Q_COUNT)[1 + 6 * warp + 1] = 32u;  // the warp has no tile yet
+  __syncwarp();
   Ctr<Count> cnt;
-  // warp-uniform tile pool
-  int tile = 0, tileTaken = 32, tileItem = 0;
   bool poolDone = false;
-  int item = 0;  // scene of the lane's pixel
-  // lane state
-  enum { NEED = 0, TRACING = 1, DONE = 2 };
-  bool hasPixel = false;
-  int ix = 0, iy = 0, s = 0, gen = 0, kind = K_NONE, tstate = NEED;
-  bool newSample = false, mainAlive = false, shadowPending = false;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  PathRay ray, sray;
+  // the lane's trace
+  int cur = -1;  // slot of the ray it traces
   Traversal T;
-  Hit h;
-  h.hit = false;
-  // the iso-surface's hit of the current trace (Iso only); with the
-  // surface's instance first, whether its box test passed and its stream
-  bool sHit = false;
-  float sT = 0.f;
-  vec3 sP;
-  vec3h sN{0, 0, 0};
-  bool isoBox = false;
-  uint64_t isoRng = 0;
   unsigned long long cyc[3] = {0ull, 0ull, 0ull};
   // profile: traversal iterations and tracing lanes summed over them, shading
   // passes and shaded lanes summed over them (lane 0 of each warp counts)
   unsigned long long simt[4] = {0ull, 0ull, 0ull, 0ull};
-  while (true) {
-    // ---- phase 1: pixels for idle lanes (from the warp's tile), then every
-    // lane that needs one starts its next trace ----
-    const unsigned need = __ballot_sync(FULL, !hasPixel);
-    if (need != 0u && !poolDone) {
-      if (tileTaken == 32) {
-        int t = 0;
-        if (lane == 0) t = atomicAdd(pool, 1);
-        t = __shfl_sync(FULL, t, 0);
-        if (t >= numTiles) {
-          poolDone = true;
-        } else {
-          tileTaken = 0;
-          if (Batch) {  // item owning global tile t: last i with tileStart[i] <= t
-            int lo = 0, hi = numItems - 1;
-            while (lo < hi) {
-              const int mid = (lo + hi + 1) >> 1;
-              if (tileStart[mid] <= t) lo = mid;
-              else hi = mid - 1;
-            }
-            tileItem = lo;
-            tile = (int)(t - tileStart[lo]);
-          } else {
-            tile = t;
-          }
-        }
-      }
-      if (!poolDone) {
-        const RenderParams &tp = Batch ? items[tileItem] : p0;
-        // the warp tile's upper-left pixel
-        int tx, ty;
-        if (!Batch && L.numRanks > 1) {  // the k-th 32x32 tile this rank owns, 4x8 warp tiles in it
-          const long long big = (long long)L.rank + (long long)(tile >> 5) * L.numRanks;
-          const int bigX = (int)(((long long)tp.W + kRefTile - 1) / kRefTile);
-          tx = (int)(big % bigX) * kRefTile + (tile & 3) * 8;
-          ty = (int)(big / bigX) * kRefTile + ((tile >> 2) & 7) * 4;
-        } else {
-          const int tilesX = (int)(((long long)tp.W + 7) >> 3);
-          tx = (tile % tilesX) * 8;
-          ty = (tile / tilesX) * 4;
-        }
-        const int rank = __popc(need & ((1u << lane) - 1u));
-        const int take = min(__popc(need), 32 - tileTaken);
-        if (!hasPixel && rank < take) {
-          const int slot = tileTaken + rank;
-          const int px = tx + (slot & 7), py = ty + (slot >> 3);
-          if (px < tp.W && py < tp.H) {
-            hasPixel = true;
-            item = tileItem;
-            ix = px;
-            iy = py;
-            s = 0;
-            newSample = true;
-            tstate = NEED;
-            acc = L.accumIdStart == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : tp.accum[(size_t)iy * tp.W + ix];
-          }
-        }
-        tileTaken += take;
-      }
+
+  // The pass of path k is complete: the next one, or the pixel is finished.
+  auto end_pass = [&](const RenderParams &p, int k, uint32_t ctl) -> int {
+    if (ctl & F_SPLIT) {
+      if (!(ctl & F_LONE)) log_end(L, P.u(W_REC, k), P.u(W_MASK, k), 1.f);
+      return Q_FREE;
     }
-    if (poolDone && __all_sync(FULL, !hasPixel)) break;
-    const RenderParams &p = Batch ? items[item] : p0;
-    long long c0 = (Count && L.profile) ? clock64() : 0;
-    if (hasPixel && tstate == NEED) {
-      if (newSample) {
-        generate_primary(p, ix, iy, L.accumIdStart + s, ray);
-        gen = 0;
-        mainAlive = true;
-        shadowPending = false;
-        newSample = false;
-      }
-      h.hit = false;
-      kind = shadowPending ? K_SHADOW : K_MAIN;
-      RNGSeed seed = shadowPending ? sray.seed : ray.seed;
-      bool active;
-      if (Iso) {
-        const vec3 org = shadowPending ? sray.org : ray.org, dir = shadowPending ? sray.dir : ray.dir;
-        float tmax = shadowPending ? sray.tMax : ray.tMax;
-        sHit = false;
-        isoBox = false;
-        if (!p.hasVolume) GBV_COUNT(cnt, rays);
-        // the surface's instance first: its box test and stream now, its
-        // search once the volume's collision is known (iso_trace_after)
-        if (p.isoFirst) isoBox = iso_begin(p, org, dir, tmax, seed, isoRng);
-        active = p.hasVolume && trace_begin(p.F, p.G, p.rcpMc, org, dir, tmax, seed, T, cnt, p.volHash);
+    const int s = (int)P.u(W_PASS, k) + 1;
+    if (s == L.spp) p.accum[(size_t)P.u(W_IY, k) * p.W + P.u(W_IX, k)] = P.acc(k);
+    P.setu(W_PASS, k, (uint32_t)s);
+    P.setu(W_CTL, k, F_FRESH);
+    return s == L.spp ? Q_FREE : Q_START;
+  };
+  // The shadow ray of path k is traced: its fragment, then the main ray or
+  // the pass's end.
+  auto end_shadow = [&](const RenderParams &p, int k, uint32_t ctl, bool occluded) -> int {
+    if (!occluded || (ctl & F_SPLIT)) {
+      const float clampMax = 10.f * (float)(1 + L.accumIdStart + (int)P.u(W_PASS, k));
+      const vec3 frag = vmin(P.f(W_SMIS, k) * from_half(P.half3(W_STP, k)), vec3(clampMax));
+      if (ctl & F_SPLIT) {
+        log_fragment(L, P.u(W_REC, k), (int)((ctl >> 8) & 0xffu) - 1, occluded ? vec3(0.f) : frag);
       } else {
-        active = trace_begin(p.F, p.G, p.rcpMc, shadowPending ? sray.org : ray.org, shadowPending ? sray.dir : ray.dir,
-                             shadowPending ? sray.tMax : ray.tMax, seed, T, cnt);
+        float4 acc = P.acc(k);
+        accum_add(acc, frag);
+        P.setacc(k, acc);
       }
-      if (shadowPending) sray.seed = seed;
-      else ray.seed = seed;
-      tstate = active ? TRACING : DONE;
     }
-    // ---- phase 2: traverse while enough of the warp's busy lanes trace ----
-    long long c1 = 0;
-    if (Count && L.profile) {
-      __syncwarp();
-      c1 = clock64();
-      if (lane == 0) cyc[0] += (unsigned long long)(c1 - c0);
+    if (!(ctl & F_ALIVE)) return end_pass(p, k, ctl);
+    P.setu(W_CTL, k, ctl & ~F_SHADOW);
+    return (int)Q_READY;
+  };
+  // The volume is traced for the ray of path k (hit: at t, colour rgb).
+  auto end_trace = [&](const RenderParams &p, int k, bool hit, float t, vec3 rgb) -> int {
+    const uint32_t ctl = P.u(W_CTL, k);
+    const bool search = Iso && (!p.isoFirst || (ctl & F_ISOBOX));
+    if (ctl & F_SHADOW) {
+      // an occluded shadow ray stays so whatever the surface does
+      return search && !hit ? (int)Q_ISO : end_shadow(p, k, ctl, hit);
     }
-    {
-      const int busy = __popc(__ballot_sync(FULL, hasPixel));
+    if (hit) {
+      P.setf(W_HT, k, t);
+      P.setv3(W_HRGB, k, rgb);
+      if (Iso) P.setu(W_CTL, k, ctl | F_VOLHIT);
+    }
+    return search ? (int)Q_ISO : hit ? (int)Q_HIT : (int)Q_START;
+  };
+
+  int idle = 0;  // polls without work
+  while (true) {
+    // ---- choose a stage ----
+    const int nStart = P.waiting(Q_START), nHit = P.waiting(Q_HIT), nReady = P.waiting(Q_READY);
+    const int nIso = Iso ? P.waiting(Q_ISO) : 0;
+    const int nFree = poolDone ? 0 : P.waiting(Q_FREE);
+    const int held = __popc(__ballot_sync(FULL, cur >= 0));
+    const int nTrace = nReady + held, nOpen = nStart + nFree;
+    enum { S_NONE, S_TRACE, S_HIT, S_START, S_ISO };
+    int stage;
+    const int most = max(max(nHit, nOpen), nIso);
+    bool shading = P.shading();
+    if (shading && most < kFull) {
+      P.set_shading(0u);
+      shading = false;
+    }
+    if (most >= kFull && (shading || nTrace < kFull)) stage = nHit == most ? S_HIT : Iso && nIso == most ? S_ISO : S_START;
+    else if (nTrace >= most) stage = nTrace ? S_TRACE : S_NONE;
+    else stage = nHit == most ? S_HIT : Iso && nIso == most ? S_ISO : S_START;
+    if (stage == S_NONE) {
+      // Nothing waits: the block is done, or its paths are with other warps.
+      // Those go on with what becomes of them, so a warp may leave; it looks
+      // again for a while to share what comes.
+      if ((poolDone && P.waiting(Q_FREE) == L.slots) || ++idle > kIdlePolls) break;
+      __nanosleep(200);
+      continue;
+    }
+    idle = 0;
+    const long long c0 = (Count && L.profile) ? clock64() : 0;
+    int phase;
+    if (stage == S_TRACE) {
+      // ---- trace: seek and sample until too few lanes are left ----
+      phase = 1;
       while (true) {
-        const int tracing = __popc(__ballot_sync(FULL, tstate == TRACING));
-        if (tracing == 0 || tracing * 100 < busy * L.threshold) break;
+        unsigned act = __ballot_sync(FULL, cur >= 0);
+        const int idleLanes = 32 - __popc(act);
+        int ended = -1;  // path whose volume trace ended in this iteration
+        bool endHit = false;
+        vec3 rgb(0.f);
+        // refill in batches: the ray set-up runs for the new rays alone
+        int more = 0;
+        if (idleLanes > 0) {
+          more = P.waiting(Q_READY);
+          if (min(more, idleLanes) < (idleLanes > 24 ? 1 : kRefillMin)) more = -more;
+        }
+        if (more > 0) {
+          int n;
+          const int got = P.take(Q_READY, idleLanes, rot, n);
+          const int k = __shfl_sync(FULL, got, __popc(~act & lt));
+          if (cur < 0 && __popc(~act & lt) < n) {
+            const uint32_t ctl = P.u(W_CTL, k);
+            const bool shadow = ctl & F_SHADOW;
+            const RenderParams &p = Batch ? items[P.u(W_ITEM, k)] : p0;
+            const int o = shadow ? W_SORG : W_ORG, sw = shadow ? W_SSEED : W_SEED;
+            const vec3 org = P.v3(o, k), dir = P.v3(o + 3, k);
+            const float tmax = shadow ? P.f(W_STMAX, k) : (ctl & 0xff00u) ? INF : 1e30f;
+            RNGSeed seed;
+            seed.state = P.u64(sw, k);
+            if (Iso) {
+              uint32_t isoBit = 0;
+              if (p.isoFirst) {
+                // the surface's instance first: its box test and stream now, its
+                // search once the volume's collision is known (iso_trace_after)
+                uint64_t isoRng = 0;
+                if (iso_begin(p, org, dir, tmax, seed, isoRng)) {
+                  isoBit = F_ISOBOX;
+                  P.setu64(W_ISORNG, k, isoRng);
+                }
+              }
+              if (!p.hasVolume) GBV_COUNT(cnt, rays);
+              P.setu(W_CTL, k, (ctl & ~(F_ISOBOX | kHitMask)) | isoBit);
+            }
+            const bool active = (!Iso || p.hasVolume) &&
+                                trace_begin(p.F, p.G, p.rcpMc, org, dir, tmax, seed, T, cnt,
+                                            Iso ? p.volHash : kVolumeStreamHash);
+            P.setu64(sw, k, seed.state);
+            if (active) cur = k;
+            else ended = k;
+          }
+          act = __ballot_sync(FULL, cur >= 0);
+        }
+        if (cur >= 0) {
+          const RenderParams &p = Batch ? items[P.u(W_ITEM, cur)] : p0;
+          if (T.inCell != 2 && trace_seek(p.G, T, cnt, L.skip, !Batch && L.maskWords > 0, L.capFlag) == TR_MISS)
+            ended = cur;
+          __syncwarp(act);  // the lanes with a position sample together
+          if (T.inCell == 2) {
+            Hit h;
+            if (trace_sample(p.F, make_store<Store>(p), p.xf, T, h, cnt) == TR_HIT) {
+              ended = cur;
+              endHit = true;
+              rgb = h.rgb;
+            }
+          }
+        }
         if (Count && L.profile && lane == 0) {
           simt[0]++;
-          simt[1] += (unsigned)tracing;
+          simt[1] += __popc(act);
         }
-        if (tstate == TRACING && T.inCell != 2 &&
-            trace_seek(p.G, T, cnt, L.skip, !Batch && L.maskWords > 0, L.capFlag) == TR_MISS)
-          tstate = DONE;
-        if (tstate == TRACING && T.inCell == 2 && trace_sample(p.F, make_store<Store>(p), p.xf, T, h, cnt) == TR_HIT)
-          tstate = DONE;
-      }
-    }
-    // ---- phase 3: shade the finished traces (bounce(), shadeRays.cu:477-878) ----
-    long long c2 = 0;
-    if (Count && L.profile) {
-      __syncwarp();
-      c2 = clock64();
-      if (lane == 0) cyc[1] += (unsigned long long)(c2 - c1);
-    }
-    if (Count && L.profile) {
-      const unsigned shading = __popc(__ballot_sync(FULL, tstate == DONE));
-      if (lane == 0 && shading) {
-        simt[2]++;
-        simt[3] += shading;
-      }
-    }
-    if (Iso && tstate == DONE && p.isoFirst && isoBox) {
-      // the surface's search, up to the volume's first collision
-      PathRay &r = kind == K_SHADOW ? sray : ray;
-      sHit = iso_trace_after<Store>(p, r.org, r.dir, r.tMax, h.hit ? h.t : __int_as_float(0x7f800000), isoRng, sT,
-                                    sP, sN);
-      if (sHit) h.hit = false;
-    }
-    if (Iso && tstate == DONE && p.hasVolume && !p.isoFirst) {
-      // the iso-surface after the volume, up to the volume's hit
-      PathRay &r = kind == K_SHADOW ? sray : ray;
-      sHit = iso_trace<Store>(p, r.org, r.dir, h.hit ? h.t : r.tMax, r.seed, sT, sP, sN);
-      if (sHit) h.hit = false;
-    }
-    if (tstate == DONE) {
-      // Env-map texels: a main ray's miss lookup (radianceFromEnv) and a
-      // hit's env light sample (EnvMap::sample) each form their texture
-      // coordinates first; then one call fetches the texels of all lanes
-      // that need one, instead of one call per kind of lane.
-      Random rnd;
-      EnvPick pick;
-      float2 uv = make_float2(0.f, 0.f);
-      bool needTex = false;
-      const bool anyHit = h.hit || (Iso && sHit);
-      if (kind == K_MAIN) {
-        if (anyHit) {
-          rnd = Random::derive(ray.seed, (uint64_t)hit_hash(h.hit ? h.t : sT));
-          if (p.hasEnv) {
-            pick = Batch ? env_pick_coords_ool(p, rnd) : env_pick_coords(p, rnd);
-            uv = make_float2(pick.sx, pick.sy);
-            needTex = true;
+        if (ended >= 0) {
+          P.publish(end_trace(Batch ? items[P.u(W_ITEM, ended)] : p0, ended, endHit, T.t, rgb), ended);
+          if (ended == cur) cur = -1;
+        }
+        const int n = __popc(__ballot_sync(FULL, cur >= 0));
+        if (more == 0 && n == 0) break;
+        const bool low = more <= 0 && n * 100 < 32 * L.threshold;
+        if (low || P.shading()) {
+          if (P.waiting(Q_HIT) >= kFull || P.waiting(Q_START) >= kFull || (Iso && P.waiting(Q_ISO) >= kFull)) {
+            P.set_shading(1u);
+            break;
           }
-        } else if (p.hasEnv) {
-          uv = Batch ? env_miss_coords_ool(p, ray.dir) : env_miss_coords(p, ray.dir);
-          needTex = true;
         }
       }
-      vec3 texel(0.f);
-      if (needTex) {
-        const float4 t = Batch ? tex2D_ool(p.env, uv.x, uv.y) : tex2D(p.env, uv.x, uv.y);
-        texel = p.env.scale * vec3(t.x, t.y, t.z);
+    } else if (stage == S_HIT) {
+      // ---- shade hits (bounce(), shadeRays.cu:477-878) ----
+      phase = 2;
+      int n;
+      const int k = P.take(Q_HIT, 32, rot, n);
+      if (Count && L.profile && lane == 0) {
+        simt[2]++;
+        simt[3] += n;
       }
-      tstate = NEED;
-      const int accumID = L.accumIdStart + s;
-      const float clampMax = 10.f * (float)(1 + accumID);
-      if (kind == K_SHADOW) {
-        if (!anyHit) accum_add(acc, vmin(sray.misWeight * from_half(sray.tp), vec3(clampMax)));
-        shadowPending = false;
-      } else {
+      ShadeOut so;
+      uint32_t ctl = 0u;
+      bool shadow = false;
+      if (k >= 0) {
+        const RenderParams &p = Batch ? items[P.u(W_ITEM, k)] : p0;
+        ctl = P.u(W_CTL, k);
+        const int gen = (int)((ctl >> 8) & 0xffu);
+        PathRay ray;
+        ray.org = P.v3(W_ORG, k);
+        ray.dir = P.v3(W_DIR, k);
+        ray.seed.state = P.u64(W_SEED, k);
+        ray.tp = P.half3(W_TP, k);
+        const uint32_t bounces = P.u(W_TP + 1, k) >> 16;
+        ray.numVolumeBounces = (int)(bounces & 0xffu);
+        ray.numDiffuseBounces = (int)(bounces >> 8);
+        ray.misWeight = P.f(W_MIS, k);
+        ray.tMax = 1.f;
+        Hit h;
+        h.hit = !Iso || !(ctl & F_SURFHIT);
+        h.t = P.f(W_HT, k);
+        h.rgb = P.v3(W_HRGB, k);
+        Random rnd = Random::derive(ray.seed, (uint64_t)hit_hash(h.t));
+        EnvPick pick;
+        if (p.hasEnv) {
+          pick = env_pick_coords(p, rnd);
+          const float4 t = tex2D(p.env, pick.sx, pick.sy);
+          pick.radiance = p.env.scale * vec3(t.x, t.y, t.z);
+        }
+        const int accumID = L.accumIdStart + (int)P.u(W_PASS, k);
         if (!Batch && gen == 0 && (p.depth || p.primId || p.instId || p.objId))
-          write_aux(p, (size_t)iy * p.W + ix, accumID, !anyHit ? ray.tMax : h.hit ? h.t : sT,
-                    !anyHit ? 0 : h.hit ? 1 : 2);
-        vec3 frag(0.f);
-        float alpha = 0.f;
-        if (!anyHit) {
+          write_aux(p, (size_t)P.u(W_IY, k) * p.W + P.u(W_IX, k), accumID, h.t, h.hit ? 1 : 2);
+        // a hit's own fragment is zero; the first generation's alpha is one
+        if (gen == 0 && !(ctl & F_SPLIT)) {
+          if (accumID == 0) P.setacc(k, make_float4(0.f, 0.f, 0.f, 1.f));
+          else P.setf(W_ACC + 3, k, P.f(W_ACC + 3, k) + 1.f);
+        }
+        // setVolumeHit's P = obj_org + t * obj_dir (MCAccelerator.h:79), the
+        // trace direction's zero components replaced as trace_begin does
+        vec3 tdir = ray.dir;
+        if (tdir.x == 0.f) tdir.x = 1e-6f;
+        if (tdir.y == 0.f) tdir.y = 1e-6f;
+        if (tdir.z == 0.f) tdir.z = 1e-6f;
+        const vec3 hitP = ray.org + h.t * tdir;
+        if (Iso && !h.hit) bounce_surface_hit(p, ray, P.half3(W_HN, k), h.t, hitP, gen, rnd, pick, so);
+        else bounce_volume_hit(p, ray, h, hitP, gen, rnd, pick, so);
+        shadow = so.shadowValid && so.shadow.tMax > 0.f;
+        const bool alive = ray.tMax > 0.f;
+        if (alive) {
+          P.setv3(W_ORG, k, ray.org);
+          P.setv3(W_DIR, k, ray.dir);
+          P.setu64(W_SEED, k, ray.seed.state);
+          P.sethalf3(W_TP, k, ray.tp, (uint32_t)ray.numVolumeBounces | ((uint32_t)ray.numDiffuseBounces << 8));
+          P.setf(W_MIS, k, ray.misWeight);
+        }
+        ctl = (ctl & F_SPLIT) | (shadow ? F_SHADOW : 0u) | (alive ? F_ALIVE : 0u) | ((uint32_t)(gen + 1) << 8);
+        if ((ctl & F_SPLIT) && shadow) P.setu(W_MASK, k, P.u(W_MASK, k) | (1u << gen));
+      }
+      // A split path's shadow ray is traced beside its bounce ray when a slot
+      // is free for it (the log orders their fragments).
+      const bool lone = (ctl & (F_SPLIT | F_SHADOW | F_ALIVE)) == (F_SPLIT | F_SHADOW | F_ALIVE) && k >= 0;
+      const unsigned wants = __ballot_sync(FULL, lone);
+      int home = k;  // the slot of the shadow ray
+      if (wants) {
+        int m;
+        const int got = P.take(Q_FREE, __popc(wants), rot, m);
+        const int r = __popc(wants & lt);
+        const int slot = __shfl_sync(FULL, got, r);
+        if (lone && r < m) {
+          home = slot;
+          P.setu(W_REC, home, P.u(W_REC, k));
+          P.setu(W_PASS, home, P.u(W_PASS, k));
+          if (Batch) P.setu(W_ITEM, home, P.u(W_ITEM, k));
+          P.setu(W_CTL, home, (ctl & ~F_ALIVE) | F_LONE);
+          ctl &= ~F_SHADOW;
+        }
+      }
+      if (k >= 0) {
+        if (shadow) {
+          P.setv3(W_SORG, home, so.shadow.org);
+          P.setv3(W_SDIR, home, so.shadow.dir);
+          P.setf(W_STMAX, home, so.shadow.tMax);
+          P.setu64(W_SSEED, home, so.shadow.seed.state);
+          P.sethalf3(W_STP, home, so.shadow.tp);
+          P.setf(W_SMIS, home, so.shadow.misWeight);
+        }
+        if (home != k) P.publish(Q_READY, home);
+        int q = Q_READY;
+        if (ctl & (F_SHADOW | F_ALIVE)) P.setu(W_CTL, k, ctl);
+        else q = end_pass(Batch ? items[P.u(W_ITEM, k)] : p0, k, ctl);
+        P.publish(q, k);
+      }
+    } else if (stage == S_START) {
+      // ---- start passes (_generateRays) and shade misses ----
+      // A new primary ray that misses the field's bounds is shaded at once,
+      // and a warp most of whose paths end this way (background) goes on with
+      // their next passes.  Free slots take new pixels.
+      phase = 0;
+      int n;
+      int k = nStart ? P.take(Q_START, 32, rot, n) : (n = 0, -1);
+      bool mine = k >= 0, fresh = false, outer = false;
+      int ix = 0, iy = 0, s = 0, gen = 0, item = 0;
+      uint32_t split = 0u, rec = 0u, mask = 0u;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      vec3 dir(0.f), weight(0.f);  // weight: the path's throughput (later generations)
+      float mis = 0.f;
+      if (mine) {
+        const uint32_t ctl = P.u(W_CTL, k);
+        fresh = ctl & F_FRESH;
+        split = ctl & F_SPLIT;
+        outer = ctl & F_OUTER;
+        ix = (int)P.u(W_IX, k);
+        iy = (int)P.u(W_IY, k);
+        s = (int)P.u(W_PASS, k);
+        acc = P.acc(k);
+        rec = P.u(W_REC, k);
+        mask = P.u(W_MASK, k);
+        if (Batch) item = (int)P.u(W_ITEM, k);
+        if (!fresh) {
+          gen = (int)((ctl >> 8) & 0xffu);
+          dir = P.v3(W_DIR, k);
+          weight = from_half(P.half3(W_TP, k));
+          mis = P.f(W_MIS, k);
+        }
+      }
+      if (n < 32 && !poolDone) {
+        int m;
+        const int got = P.take(Q_FREE, 32 - n, rot, m);
+        const int slot = __shfl_sync(FULL, got, lane - n);
+        if (lane >= n && lane < n + m) k = slot;
+      }
+      // the warp's tile, kept in shared memory between its visits here
+      uint32_t *const own = P.queue(Q_COUNT) + 1 + 6 * warp;
+      int tile = (int)own[0], tileTaken = (int)own[1], tileItem = (int)own[2], tilePass = (int)own[3];
+      uint32_t tileRec = own[4];  // log record of a split tile's first pixel
+      bool tileSplit = own[5] & 1u, tileOuter = own[5] & 2u;
+      while (true) {
+        // pixels for the lanes that hold a free slot
+        while (true) {
+          const unsigned need = __ballot_sync(FULL, k >= 0 && !mine);
+          if (!need || poolDone) break;
+          if (tileTaken == 32) {
+            int t = 0;
+            if (lane == 0) t = atomicAdd(pool, 1);
+            t = __shfl_sync(FULL, t, 0);
+            if (t >= launch_tiles(L)) {
+              poolDone = true;
+              break;
+            }
+            tileTaken = 0;
+            tilePass = 0;
+            long long idx = t;
+            const long long j = t - L.whole;
+            tileOuter = j >= L.split * L.spp;
+            tileSplit = j >= 0 && !tileOuter;
+            if (tileSplit) {
+              tileRec = (uint32_t)j * 32u;
+              tilePass = (int)((uint32_t)j % (uint32_t)L.spp);
+              idx = L.whole + (uint32_t)j / (uint32_t)L.spp;
+            } else if (tileOuter) {
+              idx = j - L.split * L.spp;
+            }
+            if (Batch) {  // the item whose tiles idx falls in
+              const long long *start = tileOuter ? tileStart + numItems + 1 : tileStart;
+              tileItem = tile_item(start, numItems, idx);
+              idx -= start[tileItem];
+            }
+            const RenderParams &tp = Batch ? items[tileItem] : p0;
+            tile = tileOuter ? outer_tile(tp, (int)idx) : inner_tile(tp, (int)idx);
+          }
+          const RenderParams &tp = Batch ? items[tileItem] : p0;
+          int tx, ty;
+          tile_corner<Batch>(L, tp, tile, tx, ty);
+          const int r = __popc(need & lt), take = min(__popc(need), 32 - tileTaken);
+          if (k >= 0 && !mine && r < take) {
+            const int at = tileTaken + r;
+            const int px = tx + (at & 7), py = ty + (at >> 3);
+            if (px < tp.W && py < tp.H) {
+              mine = fresh = true;
+              ix = px;
+              iy = py;
+              s = tilePass;
+              split = tileSplit ? F_SPLIT : 0u;
+              outer = tileOuter;
+              rec = tileRec + (uint32_t)at;
+              mask = 0u;
+              acc = L.accumIdStart == 0 || tileSplit ? make_float4(0.f, 0.f, 0.f, 0.f)
+                                                     : tp.accum[(size_t)py * tp.W + px];
+              item = tileItem;
+            }
+          }
+          tileTaken += take;
+        }
+        const RenderParams &p = Batch ? items[item] : p0;
+        bool missed = mine && !fresh;
+        if (mine && fresh) {
+          // a pixel outside the rectangle sees nothing of the field: its ray
+          // matters to the env map alone
+          PathRay ray;
+          bool enters = false;
+          gen = 0;
+          if (!outer || p.hasEnv) generate_primary(p, ix, iy, L.accumIdStart + s, ray);
+          if (!outer) {
+            vec3 tdir = ray.dir;
+            if (tdir.x == 0.f) tdir.x = 1e-6f;
+            if (tdir.y == 0.f) tdir.y = 1e-6f;
+            if (tdir.z == 0.f) tdir.z = 1e-6f;
+            float tLo = 0.f, tHi = ray.tMax;
+            enters = box_test(ray.org, tdir, tLo, tHi, p.F.boundsLo, p.F.boundsHi);
+          }
+          if (enters) {
+            P.setv3(W_ORG, k, ray.org);
+            P.setv3(W_DIR, k, ray.dir);
+            P.setu64(W_SEED, k, ray.seed.state);
+            P.sethalf3(W_TP, k, ray.tp);
+            P.setf(W_MIS, k, ray.misWeight);
+            if (split) {
+              P.setu(W_REC, k, rec);
+              P.setu(W_MASK, k, 0u);
+            } else {
+              P.setacc(k, acc);
+            }
+            P.setu(W_PASS, k, (uint32_t)s);
+            P.setu(W_IX, k, (uint32_t)ix);
+            P.setu(W_IY, k, (uint32_t)iy);
+            if (Batch) P.setu(W_ITEM, k, (uint32_t)item);
+            P.setu(W_CTL, k, F_ALIVE | split);
+            P.publish(Q_READY, k);
+            mine = false;
+            k = -1;
+          } else {
+            GBV_COUNT(cnt, rays);
+            dir = ray.dir;
+            missed = true;
+          }
+        }
+        if (missed) {
+          const int accumID = L.accumIdStart + s;
+          if (!Batch && gen == 0 && (p.depth || p.primId || p.instId || p.objId))
+            write_aux(p, (size_t)iy * p.W + ix, accumID, 1e30f, 0);
+          vec3 env(0.f);
+          if (p.hasEnv) {
+            const float2 uv = env_miss_coords(p, dir);
+            const float4 t = tex2D(p.env, uv.x, uv.y);
+            env = p.env.scale * vec3(t.x, t.y, t.z);
+          } else if (gen != 0) {
+            env = vec3(p.ambient);
+          }
           const float4 miss = miss_color(p, iy);
-          const vec3 env = p.hasEnv ? texel : (gen != 0 ? vec3(p.ambient) : vec3(0.f));
+          vec3 frag;
+          float alpha = 0.f;
           if (gen == 0) {
             alpha = miss.w;
             frag = p.hasEnv ? env : vec3(miss.x, miss.y, miss.z);
           } else {
-            frag = from_half(ray.tp) * env * ray.misWeight;
+            frag = weight * env * mis;
           }
-          ray.tMax = -1.f;
-        } else {
-          if (gen == 0) alpha = 1.f;
-          ShadeOut so;
-          // setVolumeHit's P = obj_org + t * obj_dir (MCAccelerator.h:79)
-          pick.radiance = texel;
-          if (Iso && !h.hit)
-            bounce_surface_hit(p, ray, sN, sT, sP, gen, rnd, pick, so);
-          else if (Batch)
-            bounce_volume_hit_ool(p, ray, h, T.org + h.t * T.dir, gen, rnd, pick, so);
-          else
-            bounce_volume_hit(p, ray, h, T.org + h.t * T.dir, gen, rnd, pick, so);
-          if (so.shadowValid && so.shadow.tMax > 0.f) {
-            sray = so.shadow;
-            shadowPending = true;
+          frag = vmin(frag, vec3(10.f * (float)(1 + accumID)));
+          if (split) {
+            log_fragment(L, rec, gen, frag);
+            log_end(L, rec, mask | (1u << gen) | (gen == 0 ? kLogMissed : 0u), gen == 0 ? alpha : 1.f);
+            mine = false;
+          } else {
+            if (accumID == 0 && gen == 0) {
+              acc = make_float4(frag.x, frag.y, frag.z, alpha);
+            } else {
+              if (gen == 0 && alpha > 0.f) acc.w += alpha;
+              accum_add(acc, frag);
+            }
+            if (++s == L.spp) {
+              p.accum[(size_t)iy * p.W + ix] = acc;
+              mine = false;
+            }
           }
+          fresh = true;
         }
-        frag = vmin(frag, vec3(clampMax));
-        if (accumID == 0 && gen == 0) {
-          acc = make_float4(frag.x, frag.y, frag.z, alpha);
-        } else {
-          if (gen == 0 && alpha > 0.f) acc.w += alpha;
-          accum_add(acc, frag);
-        }
-        mainAlive = ray.tMax > 0.f;
-        gen++;
+        if (__popc(__ballot_sync(FULL, mine || (k >= 0 && !poolDone))) < kRepeatMin) break;
       }
-      if (!shadowPending && !mainAlive) {
-        // this pixel's pass is complete
-        if (++s == L.spp) {
-          p.accum[(size_t)iy * p.W + ix] = acc;
-          hasPixel = false;
-        } else {
-          newSample = true;
-        }
-      }
-    }
-    if (Count && L.profile) {
       __syncwarp();
-      if (lane == 0) cyc[2] += (unsigned long long)(clock64() - c2);
+      if (lane == 0) {
+        own[0] = (uint32_t)tile;
+        own[1] = (uint32_t)tileTaken;
+        own[2] = (uint32_t)tileItem;
+        own[3] = (uint32_t)tilePass;
+        own[4] = tileRec;
+        own[5] = (tileSplit ? 1u : 0u) | (tileOuter ? 2u : 0u);
+      }
+      if (mine) {
+        P.setacc(k, acc);
+        P.setu(W_PASS, k, (uint32_t)s);
+        P.setu(W_IX, k, (uint32_t)ix);
+        P.setu(W_IY, k, (uint32_t)iy);
+        if (Batch) P.setu(W_ITEM, k, (uint32_t)item);
+        P.setu(W_CTL, k, F_FRESH | (outer ? F_OUTER : 0u));
+      }
+      if (k >= 0) P.publish(mine ? Q_START : Q_FREE, k);
+    } else {
+      // ---- the iso-surface's search, after the volume's trace ----
+      phase = 2;
+      int n;
+      const int k = P.take(Q_ISO, 32, rot, n);
+      if (k >= 0) {
+        const RenderParams &p = p0;
+        const uint32_t ctl = P.u(W_CTL, k);
+        const bool shadow = ctl & F_SHADOW, volHit = ctl & F_VOLHIT;
+        const int o = shadow ? W_SORG : W_ORG, sw = shadow ? W_SSEED : W_SEED;
+        const vec3 org = P.v3(o, k), dir = P.v3(o + 3, k);
+        const float tmax = shadow ? P.f(W_STMAX, k) : (ctl & 0xff00u) ? INF : 1e30f;
+        float sT = 0.f;
+        vec3 sP;
+        vec3h sN{0, 0, 0};
+        bool hit;
+        if (p.isoFirst) {
+          // the surface's search, up to the volume's first collision
+          hit = iso_trace_after<Store>(p, org, dir, tmax, volHit ? P.f(W_HT, k) : INF, P.u64(W_ISORNG, k), sT, sP, sN);
+        } else {
+          // the iso-surface after the volume, up to the volume's hit
+          RNGSeed seed;
+          seed.state = P.u64(sw, k);
+          hit = iso_trace<Store>(p, org, dir, volHit ? P.f(W_HT, k) : tmax, seed, sT, sP, sN);
+          P.setu64(sw, k, seed.state);
+        }
+        int q;
+        if (shadow) {
+          q = end_shadow(p, k, ctl, hit);
+        } else {
+          if (hit) {
+            P.setf(W_HT, k, sT);
+            P.sethalf3(W_HN, k, sN);
+            P.setu(W_CTL, k, (ctl & ~kHitMask) | F_SURFHIT);
+          }
+          q = hit || volHit ? Q_HIT : Q_START;
+        }
+        P.publish(q, k);
+      }
     }
+    __syncwarp();
+    if (Count && L.profile && lane == 0) cyc[phase] += (unsigned long long)(clock64() - c0);
   }
   if (Count && L.counters) {
     unsigned long long v[12] = {cnt.samples, cnt.mcs, cnt.rays, cnt.caps, cnt.cells, cyc[0], cyc[1], cyc[2],
@@ -1541,6 +2032,138 @@ __global__ void __launch_bounds__(kThreads, MinBlocks)
   }
 }
 
+// Adds up the logged fragments of the split tiles: one thread per pixel,
+// pass by pass and generation by generation.
+template <bool Batch>
+static __global__ void __launch_bounds__(256) resolve_kernel(const __grid_constant__ RenderParams L,
+                                                             const RenderParams *__restrict__ items,
+                                                             const long long *__restrict__ tileStart, int numItems) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >> 5 >= L.split) return;
+  const long long t = L.whole + (i >> 5);
+  const int item = Batch ? tile_item(tileStart, numItems, t) : 0;
+  const RenderParams &p = Batch ? items[item] : L;
+  const int at = (int)(i & 31);
+  int tx, ty;
+  tile_corner<Batch>(L, p, inner_tile(p, (int)(Batch ? t - tileStart[item] : t)), tx, ty);
+  tx += at & 7;
+  ty += at >> 3;
+  if (tx >= p.W || ty >= p.H) return;
+  float4 *out = p.accum + (size_t)ty * p.W + tx;
+  float4 acc = L.accumIdStart == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *out;
+  const int words = log_words(L.logHits);
+  const uint32_t *r = L.log + ((size_t)(i >> 5) * L.spp * 32 + at) * words;
+  for (int s = 0; s < L.spp; s++, r += (size_t)32 * words) {
+    uint32_t mask = r[0];
+    const float alpha = __uint_as_float(r[1]);
+    const float *f = reinterpret_cast<const float *>(r + 2);
+    if (L.accumIdStart + s == 0) {
+      acc = make_float4(0.f, 0.f, 0.f, alpha);
+      if (mask & kLogMissed) {
+        acc.x = f[0];
+        acc.y = f[1];
+        acc.z = f[2];
+        continue;
+      }
+    } else if (alpha > 0.f) {
+      acc.w += alpha;
+    }
+    for (mask &= ~kLogMissed; mask; mask &= mask - 1) {
+      const float *g = f + 3 * (__ffs(mask) - 1);
+      accum_add(acc, vec3(g[0], g[1], g[2]));
+    }
+  }
+  *out = acc;
+}
+
+// Fragments a path of this world can log: one per hit (its shadow ray) or
+// the miss that ends it.  A volume hit of the single-scatter build ends the
+// path; with isotropic scattering every hit ends it or counts against
+// maxVolumeBounces; else (a scatter of vanishing pdf leaves the ray alive and
+// counts nothing) only the path depth (10) bounds the hits.
+inline int path_hits(const RenderParams &p) {
+  if (p.isoOn || (p.multi && !(fabsf(p.aniso) < 1e-3f))) return 11;
+  if (!p.multi || !p.volMS) return 1;
+  return p.maxVB < 0 ? 1 : p.maxVB < 10 ? p.maxVB + 1 : 11;
+}
+// Log memory of a launch at most
+constexpr size_t kLogBytes = (size_t)256 << 20;
+constexpr int kBatchLogPasses = 16;
+// The rectangle of warp tiles the field's bounds project to (p.rx, ...);
+// returns the number of tiles in it.  A tile outside it provably sees nothing
+// of the field: the bounds' projection is the hull of its corners'
+// projections, taken here in double, and the tile's pixels keep a margin of
+// two pixels from the hull's rectangle, at least 2e-5 rad where a pixel spans
+// 1e-5 rad or more.  A ray's float direction is within 1e-6 rad of its exact
+// one, and rotating a ray by d changes the ratio of two slab distances by
+// sqrt(2) d or more, against a rounding error of 1e-6 in the float slab test.
+// Where that does not hold (a corner behind or beside the camera, finer
+// pixels, values that are not finite) the rectangle is the whole frame.  A
+// launch of a rank's share of the tiles has no rectangle: rw = 0, every tile
+// is an inner one.
+inline long long plan_rect(RenderParams &p) {
+  const long long tx = ((long long)p.W + 7) >> 3, ty = ((long long)p.H + 3) >> 2;
+  p.rx = p.ry = p.rw = p.rh = 0;
+  if (p.numRanks > 1) return warp_tile_count(p);
+  struct D3 { double x, y, z; };
+  auto dotd = [](D3 a, vec3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; };
+  const double aspect = (double)p.W / p.H;
+  const D3 d00{p.dir00.x, p.dir00.y, p.dir00.z};
+  const double dd = dotd(d00, p.dir00);  // dir00 is 1 / (2 tan(fovy / 2)) long, du and dv are unit vectors
+  // the smallest angle a pixel spans, at the frame's corners
+  const double corner2 = dd + .25 * aspect * aspect + .25;
+  bool whole = !(sqrt(dd) / corner2 / p.H > 1e-5);
+  double x0 = 1e30, x1 = -1e30, y0 = 1e30, y1 = -1e30;
+  for (int k = 0; k < 8 && !whole; k++) {
+    const D3 d{(double)(k & 1 ? p.F.boundsHi.x : p.F.boundsLo.x) - p.lens00.x,
+               (double)(k & 2 ? p.F.boundsHi.y : p.F.boundsLo.y) - p.lens00.y,
+               (double)(k & 4 ? p.F.boundsHi.z : p.F.boundsLo.z) - p.lens00.z};
+    const double t = dotd(d, p.dir00) / dd, len = sqrt(d.x * d.x + d.y * d.y + d.z * d.z);
+    whole = !(t * sqrt(dd) > 1e-3 * len);
+    const double x = (.5 + dotd(d, p.du) / t / aspect) * p.W, y = (.5 + dotd(d, p.dv) / t) * p.H;
+    whole = whole || !(fabs(x) < 1e9 && fabs(y) < 1e9);
+    x0 = x < x0 ? x : x0;
+    x1 = x > x1 ? x : x1;
+    y0 = y < y0 ? y : y0;
+    y1 = y > y1 ? y : y1;
+  }
+  if (whole) {
+    p.rw = (int)tx;
+    p.rh = (int)ty;
+    return tx * ty;
+  }
+  // tiles that overlap [x0 - 2, x1 + 2] x [y0 - 2, y1 + 2]
+  auto tiles = [](double lo, double hi, int pixels, int edge, int &first, int &count) {
+    const long long a = clampv((long long)floor(lo - 2.), 0ll, (long long)pixels) / edge;
+    const long long b = (clampv((long long)ceil(hi + 2.), 0ll, (long long)pixels) + edge - 1) / edge;
+    first = (int)a;
+    count = (int)(b - a);
+  };
+  tiles(x0, x1, p.W, 8, p.rx, p.rw);
+  tiles(y0, y1, p.H, 4, p.ry, p.rh);
+  if (p.rw <= 0 || p.rh <= 0) {  // the frame sees nothing of the field: one inner tile, so that rw > 0
+    p.rx = p.ry = 0;
+    p.rw = p.rh = 1;
+  }
+  return (long long)p.rw * p.rh;
+}
+
+// What a launch over `inner` + `outer` tiles splits: as many of the last
+// inner tiles as `room` bytes of log hold.  Returns the log's bytes.
+inline size_t plan_split(RenderParams &p, long long inner, long long outer, int hits, size_t room) {
+  const size_t perTile = (size_t)p.spp * 32 * log_words(hits) * sizeof(uint32_t);
+  long long split = (long long)(room / perTile);
+  if (split > inner) split = inner;
+  // a pixel's depth channel is the running minimum of its passes in order
+  if (p.depth || p.primId || p.instId || p.objId) split = 0;
+  if (split * 16 < inner || inner + outer + split * p.spp >= (1ll << 31) - (1ll << 24)) split = 0;
+  p.whole = inner - split;
+  p.split = split;
+  p.outer = outer;
+  p.logHits = hits;
+  p.log = nullptr;
+  return (size_t)split * perTile;
+}
 
 // 32-bit words of dynamic shared memory the staged tables take
 inline size_t staged_words(const RenderParams &p) {
@@ -1551,15 +2174,41 @@ inline size_t staged_words(const RenderParams &p) {
   return (size_t)end;
 }
 
+using RenderKernelFn = void (*)(const RenderParams, const RenderParams *, const long long *, int, int *);
+
+// Places the block's path pool behind the `staged` words of tables; returns
+// the block's dynamic shared memory in bytes.
+template <bool Iso> inline size_t plan_pool(RenderParams &p, size_t staged) {
+  p.poolOff = (int)((staged + 3) & ~(size_t)3);
+  return ((size_t)p.poolOff + PathPool<Iso>::kStride) * sizeof(uint32_t);
+}
+
+// Persistent grid of a launch over `tiles` warp tiles: one block per SM, and
+// the path slots each block uses: no more than its share of the pixels, so
+// that no block holds pixels that another would be idle without.
+inline gbv_status plan_grid(RenderParams &p, RenderKernelFn kernel, size_t smem, long long tiles, long long &blocks) {
+  int dev = 0, sms = 0;
+  gbv_status st = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+  if (st == GBV_OK) st = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+  if (st == GBV_OK && smem > 48 * 1024)
+    st = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                    "render_kernel: shared-memory size");
+  if (st != GBV_OK) return st;
+  blocks = tiles < sms ? tiles : sms;
+  if (blocks < 1) blocks = 1;
+  const long long share = 32 * ((tiles + blocks - 1) / blocks);
+  p.slots = (int)(share < kSlots ? share : kSlots);
+  return GBV_OK;
+}
+
 // The one-scene render kernels of a launch: with and without event
 // counting, for a volume-only world or (at 4 resident blocks per SM) one
 // with an iso-surface.
-using RenderKernelFn = void (*)(const RenderParams, const RenderParams *, const long long *, int, int *);
-template <class Store, int MinBlocks>
+template <class Store, int Budget>
 inline void render_kernels(const RenderParams &p, RenderKernelFn &counting, RenderKernelFn &plain) {
-  counting = render_kernel<Store, MinBlocks, false, true>;
-  plain = render_kernel<Store, MinBlocks, false, false>;
-  if constexpr (MinBlocks == 4) {
+  counting = render_kernel<Store, Budget, false, true>;
+  plain = render_kernel<Store, Budget, false, false>;
+  if constexpr (Budget == 4) {
     if (p.isoOn) {
       counting = render_kernel<Store, 4, false, true, true>;
       plain = render_kernel<Store, 4, false, false, true>;
@@ -1567,42 +2216,31 @@ inline void render_kernels(const RenderParams &p, RenderKernelFn &counting, Rend
   }
 }
 
-template <class Store, int MinBlocks>
+template <class Store, int Budget>
 inline gbv_status launch_render_t(const RenderParams &p, const Store &store, cudaStream_t stream) {
-  // persistent grid: as many resident blocks as the device holds
-  int dev = 0, sms = 0, perSM = 0;
-  gbv_status st = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
-  if (st == GBV_OK) st = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-  if (st != GBV_OK) return st;
   RenderKernelFn kCount, kPlain;
-  render_kernels<Store, MinBlocks>(p, kCount, kPlain);
-  const size_t smem = staged_words(p) * sizeof(uint32_t);
-  if (smem > 48 * 1024) {
-    st = check_cuda(cudaFuncSetAttribute(kCount, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                    "render_kernel: shared-memory size");
-    if (st == GBV_OK)
-      st = check_cuda(cudaFuncSetAttribute(kPlain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                      "render_kernel: shared-memory size");
-    if (st != GBV_OK) return st;
-  }
-  st = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kCount, kThreads, smem),
-                  "render_kernel: occupancy");
-  if (st != GBV_OK) return st;
-  const long long tiles = warp_tile_count(p);
-  const long long warpsPerBlock = kThreads / 32;
-  long long blocks = (long long)sms * (perSM > 0 ? perSM : 1);
-  const long long needed = (tiles + warpsPerBlock - 1) / warpsPerBlock;
-  if (blocks > needed) blocks = needed;
-  if (blocks < 1) blocks = 1;
+  render_kernels<Store, Budget>(p, kCount, kPlain);
+  const RenderKernelFn kernel = p.counters ? kCount : kPlain;
+  RenderParams q = p;
+  const size_t smem = p.isoOn ? plan_pool<true>(q, staged_words(p)) : plan_pool<false>(q, staged_words(p));
+  long long blocks = 0;
+  gbv_status st = GBV_OK;
   // the tile pool counter and the majorant bitmask live in stream-ordered
   // scratch memory (the mask at a 256-byte offset: 16-byte aligned for the
   // bulk copy)
   int *pool = nullptr;
-  const size_t maskBytes = (size_t)p.maskWords * 4;
-  st = check_cuda(scratch_alloc((void **)&pool, 256 + maskBytes, stream), "tile pool scratch");
+  const long long inner = plan_rect(q), outer = warp_tile_count(p) - inner;
+  size_t logBytes = plan_split(q, inner, outer, path_hits(p), kLogBytes);
+  const size_t maskBytes = ((size_t)p.maskWords * 4 + 255) & ~(size_t)255;
+  if (logBytes && scratch_alloc((void **)&pool, 256 + maskBytes + logBytes, stream) != cudaSuccess) {
+    cudaGetLastError();  // no room for the log: no tile is split
+    logBytes = plan_split(q, inner, outer, 1, 0);
+  }
+  if (!logBytes) st = check_cuda(scratch_alloc((void **)&pool, 256 + maskBytes, stream), "tile pool scratch");
   if (st != GBV_OK) return st;
+  if (logBytes) q.log = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(pool) + 256 + maskBytes);
+  st = plan_grid(q, kernel, smem, launch_tiles(q), blocks);
   st = check_cuda(cudaMemsetAsync(pool, 0, sizeof(int), stream), "render_kernel: clearing the tile pool");
-  RenderParams q = p;
   if (st == GBV_OK && p.maskWords > 0 && p.maskSrc == nullptr && p.maskMode == 0) {
     uint32_t *mask = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(pool) + 256);
     const int nmc = p.G.M[0] * p.G.M[1] * p.G.M[2];
@@ -1611,8 +2249,12 @@ inline gbv_status launch_render_t(const RenderParams &p, const Store &store, cud
     q.maskSrc = mask;
   }
   if (st == GBV_OK) {
-    (p.counters ? kCount : kPlain)<<<(unsigned)blocks, kThreads, smem, stream>>>(q, nullptr, nullptr, 0, pool);
+    kernel<<<(unsigned)blocks, block_threads(Budget), smem, stream>>>(q, nullptr, nullptr, 0, pool);
     st = check_launch("render_kernel");
+  }
+  if (st == GBV_OK && q.log) {
+    resolve_kernel<false><<<(unsigned)((q.split * 32 + 255) / 256), 256, 0, stream>>>(q, nullptr, nullptr, 0);
+    st = check_launch("resolve_kernel");
   }
   const gbv_status fst = check_cuda(cudaFreeAsync(pool, stream), "cudaFreeAsync(tile pool)");
   return st != GBV_OK ? st : fst;
@@ -1690,24 +2332,19 @@ inline gbv_status launch_render_noalloc(RenderParams p, const Store &store, cuda
   p.cdfYOff = p.pivOff = p.rowOff = -1;
   p.pivPerRow = 0;
   p.profile = 0;
-  int dev = 0, sms = 0, perSM = 0;
+  // no tile is split: a log would be an allocation
+  const long long inner = plan_rect(p);
+  plan_split(p, inner, warp_tile_count(p) - inner, 1, 0);
   RenderKernelFn kCount, kPlain;
   render_kernels<Store, 4>(p, kCount, kPlain);
-  gbv_status st = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
-  if (st == GBV_OK) st = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-  if (st == GBV_OK)
-    st = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kCount, kThreads, 0),
-                    "render_kernel: occupancy");
+  const RenderKernelFn kernel = p.counters ? kCount : kPlain;
+  const size_t smem = p.isoOn ? plan_pool<true>(p, 0) : plan_pool<false>(p, 0);
+  long long blocks = 0;
+  gbv_status st = plan_grid(p, kernel, smem, launch_tiles(p), blocks);
   if (st != GBV_OK) return st;
-  const long long tiles = warp_tile_count(p);
-  const long long warpsPerBlock = kThreads / 32;
-  long long blocks = (long long)sms * (perSM > 0 ? perSM : 1);
-  const long long needed = (tiles + warpsPerBlock - 1) / warpsPerBlock;
-  if (blocks > needed) blocks = needed;
-  if (blocks < 1) blocks = 1;
   st = check_cuda(cudaMemsetAsync(pool, 0, sizeof(int), stream), "gbv_render_noalloc: clearing the tile pool");
   if (st != GBV_OK) return st;
-  (p.counters ? kCount : kPlain)<<<(unsigned)blocks, kThreads, 0, stream>>>(p, nullptr, nullptr, 0, pool);
+  kernel<<<(unsigned)blocks, block_threads(4), smem, stream>>>(p, nullptr, nullptr, 0, pool);
   return check_launch("render_kernel (noalloc)");
 }
 
@@ -1717,47 +2354,44 @@ struct gbv_batch {
   int count;
   int format, layout;
   gbv::RenderParams *d_items;  // device copy of the per-item parameters
-  long long *d_tileStart;      // prefix sums of the items' 8x4 tile counts
+  long long *d_tileStart;      // prefix sums of the items' inner 8x4 tiles, then of their outer ones
   int *d_pool;                 // tile-pool counter
-  long long totalTiles;
+  long long innerTiles, outerTiles;
   int occ, threshold, skip;
   int device;
+  int hits;          // most fragments a path of any item can log
+  uint32_t *d_log;   // log of the split tiles (null: none are split)
+  size_t logBytes;
 };
 
 namespace gbv {
 
+template <class Store, int Budget>
+inline gbv_status batch_launch_t(const gbv_batch *b, RenderParams L, cudaStream_t stream) {
+  const RenderKernelFn kernel = L.counters ? render_kernel<Store, Budget, true, true>
+                                           : render_kernel<Store, Budget, true, false>;
+  const size_t smem = plan_pool<false>(L, 0);
+  long long blocks = 0;
+  if (plan_split(L, b->innerTiles, b->outerTiles, b->hits, b->logBytes)) L.log = b->d_log;
+  gbv_status st = plan_grid(L, kernel, smem, launch_tiles(L), blocks);
+  if (st == GBV_OK) st = check_cuda(cudaMemsetAsync(b->d_pool, 0, sizeof(int), stream), "gbv_batch_render: pool");
+  if (st != GBV_OK) return st;
+  kernel<<<(unsigned)blocks, block_threads(Budget), smem, stream>>>(L, b->d_items, b->d_tileStart, b->count, b->d_pool);
+  st = check_launch("render_kernel (batch)");
+  if (st == GBV_OK && L.log) {
+    resolve_kernel<true><<<(unsigned)((L.split * 32 + 255) / 256), 256, 0, stream>>>(L, b->d_items, b->d_tileStart,
+                                                                                     b->count);
+    st = check_launch("resolve_kernel (batch)");
+  }
+  return st;
+}
 template <class Store>
-inline gbv_status batch_launch(const gbv_batch *b, RenderParams L, cudaStream_t stream) {
-  int sms = 0, perSM = 0;
-  gbv_status st = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device), "SM count");
-  if (st != GBV_OK) return st;
-  const long long warpsPerBlock = kThreads / 32;
-  st = check_cuda(cudaMemsetAsync(b->d_pool, 0, sizeof(int), stream), "gbv_batch_render: pool");
-  if (st != GBV_OK) return st;
-#define GBV_BATCH_LAUNCH(OCC)                                                                              \
-  {                                                                                                        \
-    st = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, render_kernel<Store, OCC, true, true>, \
-                                                                  kThreads, 0),                            \
-                    "render_kernel (batch): occupancy");                                                   \
-    if (st != GBV_OK) return st;                                                                           \
-    long long blocks = (long long)sms * (perSM > 0 ? perSM : 1);                                           \
-    const long long needed = (b->totalTiles + warpsPerBlock - 1) / warpsPerBlock;                         \
-    if (blocks > needed) blocks = needed;                                                                  \
-    if (blocks < 1) blocks = 1;                                                                            \
-    if (L.counters)                                                                                        \
-      render_kernel<Store, OCC, true, true><<<(unsigned)blocks, kThreads, 0, stream>>>(                    \
-          L, b->d_items, b->d_tileStart, b->count, b->d_pool);                                             \
-    else                                                                                                   \
-      render_kernel<Store, OCC, true, false><<<(unsigned)blocks, kThreads, 0, stream>>>(                   \
-          L, b->d_items, b->d_tileStart, b->count, b->d_pool);                                             \
-  }
+inline gbv_status batch_launch(const gbv_batch *b, const RenderParams &L, cudaStream_t stream) {
   switch (b->occ) {
-    case 4: GBV_BATCH_LAUNCH(4) break;
-    case 6: GBV_BATCH_LAUNCH(6) break;
-    default: GBV_BATCH_LAUNCH(5) break;
+    case 4: return batch_launch_t<Store, 4>(b, L, stream);
+    case 6: return batch_launch_t<Store, 6>(b, L, stream);
+    default: return batch_launch_t<Store, 5>(b, L, stream);
   }
-#undef GBV_BATCH_LAUNCH
-  return check_launch("render_kernel (batch)");
 }
 
 #define GBV_DECLARE_STORE_LAUNCHERS(NAME)                                                        \

@@ -278,8 +278,8 @@ typedef struct gbv_scene {
 /* Counters written by gbv_render when d_counters != 0 (uint64 each):
    [0] density samples, [1] macrocells entered with a non-zero majorant,
    [2] rays traced, [3] loop-cap events, [4] macrocells crossed (all),
-   [5..7] SM cycles spent starting traces, traversing and shading, summed
-   over warps, [8] traversal iterations of warps and [9] tracing lanes
+   [5..7] SM cycles spent starting passes and shading misses, traversing, and
+   shading hits (with an iso-surface's search), summed over warps, [8] traversal iterations of warps and [9] tracing lanes
    summed over them, [10] shading passes of warps and [11] shaded lanes
    summed over them ([5..11] only when gbv_render_ex's config asks for a
    profile, else 0). */
@@ -314,12 +314,14 @@ gbv_status gbv_render(const gbv_scene *scene, float *d_accum, int width,
    every setting renders the identical frame.  A zero field takes its
    default, so a zero-initialised struct (or a null pointer) is the default
    launch.
-   blocks_per_sm: resident 288-thread blocks per SM the registers are capped
-     for: 4 (default; 56 registers), 5 or 6.
-   threshold_pct: a warp keeps traversing while at least this percentage of
-     its busy lanes is still tracing (1..100, default 20).
-   skip_cells: cell tests and Woodcock distance draws a lane makes per
-     traversal iteration before the warp samples (1..1024, default 6).
+   blocks_per_sm: the register budget, as resident 128-thread blocks per SM:
+     4 (default; 128 registers a thread), 5 or 6.  The persistent kernel runs
+     one block of that many threads on each SM.
+   threshold_pct: a warp keeps tracing while at least this percentage of its
+     lanes is (1..100, default 25), or while no other stage has work for it.
+   skip_cells: rounds (a cell test, a Woodcock distance draw and a step) a
+     lane makes per traversal iteration before the warp samples (1..1024,
+     default 4).
    stage: shared-memory staging, GBV_STAGE_DEFAULT (the bitmask of non-zero
      majorants, at most 8 KB, computed once per launch in HBM and copied to
      each block by one bulk copy, and the env map's per-row pdf terms),
@@ -419,14 +421,14 @@ gbv_status gbv_render_noalloc(const gbv_scene *scene, float *d_accum, int width,
    own field, TF, camera, lights and frame) rendered by one persistent launch
    whose warps take 8x4-pixel tiles from all items.  No counterpart in the
    reference (which renders one model per bnRender).
-   gbv_batch_create uploads the items' parameters (allocates and copies; call
-   it outside stream capture); gbv_batch_render is one memset and one kernel
-   launch on `stream`, so a capture of it replays as a CUDA graph;
-   gbv_batch_set_launch sets the launch shape (resident 288-thread blocks per
-   SM, 4 to 6, default 4; traversal threshold %, default 20; cell tests and
-   Woodcock distance draws per lane and traversal iteration, default 6),
-   which changes speed, never results.  Items must share the voxel format and
-   layout; each item's frame accumulates exactly as gbv_render would. */
+   gbv_batch_create uploads the items' parameters and takes up to 256 MB of
+   log memory (allocates and copies; call it outside stream capture);
+   gbv_batch_render is one memset and at most two kernel launches on `stream`,
+   so a capture of it replays as a CUDA graph; gbv_batch_set_launch sets the
+   launch shape (gbv_render_config's blocks_per_sm, threshold_pct and
+   skip_cells, 4, 25 and 64 by default), which changes speed, never results.
+   Items must share the voxel format and layout; each item's frame accumulates
+   exactly as gbv_render would. */
 typedef struct gbv_batch gbv_batch;
 gbv_status gbv_batch_create(const gbv_scene *scenes, float *const *d_accums,
                             const int *widths, const int *heights, int count,

@@ -1,0 +1,158 @@
+"""Frames whose tiles are handed out pass by pass (their fragments logged and
+added up by a second kernel) equal frames rendered whole, bit for bit.
+
+gbv_render splits every tile that may see the field while the log has room;
+gbv_render_noalloc has no log and splits none.  The sizes are the edges: one
+pixel, part of a warp tile, one tile, one tile and a column and a row, and
+frames whose log has room for part of the tiles or for none."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+from barney_gb300 import _native as N
+from barney_gb300 import scenes
+from barney_gb300.batch import GpuBatch
+from barney_gb300.device import GpuScene, _ptr, _stream
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def bits(a):
+    return np.ascontiguousarray(a, np.float32).view(np.uint32)
+
+
+def whole(g, spp, start=0, accum=None):
+    acc = g.new_accum() if accum is None else accum
+    N.check(N.lib().gbv_render_noalloc(C.byref(g.record()), _ptr(acc), g.s.width, g.s.height, start, spp, None,
+                                       _stream()), "gbv_render_noalloc")
+    return acc
+
+
+def world(kind, w, h):
+    """single / multi (isotropic) / forward (strong forward scattering, hits
+    bounded by the path depth only) / dark (negative background alpha: the
+    gradient) / iso / inside (camera in the volume: no tile is outside) /
+    away (the frame sees nothing of it) / tele (a pixel spans less than the
+    rectangle's margin allows)."""
+    s = scenes.small_scene(dims=40, spp=1, width=w, height=h)
+    if kind in ("multi", "forward", "iso"):
+        s.multi_scatter = s.volume_multi_scatter = 1
+        s.max_volume_bounces = 4
+        s.env = scenes.env_sky(64, 32)
+    if kind == "forward":
+        s.anisotropy, s.max_volume_bounces = 0.8, 20
+    if kind == "dark":
+        s.bg_color = (0.5, 0.25, 0.125, -1.0)
+    if kind == "iso":
+        s.iso, s.volume_instance = scenes.IsoSurface(value=0.5), 1
+    if kind == "inside":
+        s.cam_pos = (0.05, 0.02, 0.03)
+    if kind == "away":
+        s.cam_dir = tuple(-x for x in s.cam_dir)
+    if kind == "tele":
+        s.fovy = 0.05
+    return s
+
+
+KINDS = ["single", "multi", "forward", "dark", "iso", "inside", "away", "tele"]
+
+
+@pytest.mark.parametrize("size", [(1, 1), (7, 3), (8, 4), (9, 5), (57, 33)])
+@pytest.mark.parametrize("kind", KINDS)
+def test_split_equals_whole(cuda, kind, size):
+    """Fresh frames (the first pass overwrites) and continued ones, 1 pass and
+    several."""
+    import torch
+    g = GpuScene(world(kind, *size))
+    for spp, start in ((1, 0), (5, 0), (3, 2)):
+        base = torch.rand(size[1], size[0], 4, device="cuda")
+        a = g.render(spp=spp, accum=base.clone(), accum_id_start=start)
+        b = whole(g, spp, start, base.clone())
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(bits(a.cpu().numpy()), bits(b.cpu().numpy()))
+
+
+@pytest.mark.parametrize("kind", ["single", "dark", "inside", "away"])
+def test_split_frames_are_the_oracles(cuda, kind):
+    import torch
+    s = world(kind, 41, 23)
+    a = GpuScene(s).render(spp=4)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(bits(a.cpu().numpy()), bits(oracle.Oracle(s).render(spp=4)))
+
+
+@pytest.mark.parametrize("kind,w,h,spp", [("inside", 640, 400, 72), ("forward", 320, 200, 40), ("inside", 200, 120, 2000)])
+def test_partly_split_equals_whole(cuda, kind, w, h, spp):
+    """The log has room for part of the inner tiles (the first two) or for so
+    few of them that none is split."""
+    import torch
+    g = GpuScene(world(kind, w, h))
+    a, b = g.render(spp=spp), whole(g, spp)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(bits(a.cpu().numpy()), bits(b.cpu().numpy()))
+
+
+def test_split_batch_equals_whole(cuda):
+    """Items with and without outer tiles, with other bounds on their hits."""
+    import torch
+    sizes = [(1, 1), (9, 5), (57, 33), (64, 40), (16, 8)]
+    items = [world(k, *sizes[i % 5]) for i, k in enumerate(["single", "multi", "forward", "inside", "away", "dark"])]
+    b = GpuBatch(items)
+    for spp, start in ((1, 0), (5, 1)):
+        b.render(spp, accum_id_start=start)
+    for s, acc in zip(items, b.accums):
+        g = GpuScene(s)
+        ref = whole(g, 5, 1, whole(g, 1))
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(bits(acc.cpu().numpy()), bits(ref.cpu().numpy()))
+
+
+def test_scratch_is_safe_across_threads_and_streams(cuda):
+    """Launches on several threads and streams share the scratch pool: every
+    frame is the one a lone launch renders."""
+    import torch
+    gs = [GpuScene(world("single", 40 + 8 * i, 30)) for i in range(4)]
+    refs = [whole(g, 6).cpu().numpy() for g in gs]
+    out = [None] * 4
+    torch.cuda.synchronize()
+
+    def work(i):
+        st = torch.cuda.Stream()
+        with torch.cuda.stream(st):
+            frames = [gs[i].render(spp=6) for _ in range(8)]
+        st.synchronize()
+        out[i] = [f.cpu().numpy() for f in frames]
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for ref, frames in zip(refs, out):
+        for f in frames:
+            np.testing.assert_array_equal(bits(f), bits(ref))
+
+
+def test_captured_render_replays(cuda):
+    """A render captured in a CUDA graph (its scratch belongs to the graph)
+    replays to the same frame."""
+    import torch
+    g = GpuScene(world("single", 57, 33))
+    ref = whole(g, 3)
+    acc = g.new_accum()
+    g.render(spp=3, accum=acc)  # loads the kernels outside the capture
+    acc.zero_()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        with torch.cuda.graph(graph, stream=st):
+            g.render(spp=3, accum=acc)
+    for _ in range(2):
+        acc.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(bits(acc.cpu().numpy()), bits(ref.cpu().numpy()))
