@@ -117,8 +117,46 @@ GBV_HD float nvdb_leaf_value(uint32_t type, const unsigned char *lf, uint32_t n)
   return (float)code * nvdb_ld<float>(lf + kNvdbLeafQuantum) + nvdb_ld<float>(lf + kNvdbLeafMinimum);
 }
 
+// The leaf that holds index coordinates (x, y, z), or null where the tree
+// ends above the leaves: `value` is then the tile value or the background of
+// the whole 8^3 block.
+GBV_HD const unsigned char *nvdb_leaf(const NvdbGrid &g, int x, int y, int z, float &value) {
+  const unsigned char *root = g.base + g.root;
+  const uint64_t key = (uint64_t)((uint32_t)z >> 12) | ((uint64_t)((uint32_t)y >> 12) << 21) |
+                       ((uint64_t)((uint32_t)x >> 12) << 42);
+  const unsigned char *tile = nullptr;
+  for (uint32_t i = 0; i < g.tiles; i++) {
+    const unsigned char *t = root + kNvdbRootTiles + (size_t)kNvdbRootTile * i;
+    if (nvdb_ld<uint64_t>(t) == key) {
+      tile = t;
+      break;
+    }
+  }
+  value = g.background;
+  if (!tile) return nullptr;
+  const long long child = nvdb_ld<long long>(tile + kNvdbTileChild);
+  if (child == 0) {
+    value = nvdb_ld<float>(tile + kNvdbTileValue);
+    return nullptr;
+  }
+  const unsigned char *up = root + child;
+  uint32_t n = (((uint32_t)x & 4095u) >> 7 << 10) | (((uint32_t)y & 4095u) >> 7 << 5) | (((uint32_t)z & 4095u) >> 7);
+  if (!((nvdb_ld<uint64_t>(up + kNvdbUpperChildMask + 8 * (n >> 6)) >> (n & 63)) & 1ull)) {
+    value = nvdb_ld<float>(up + kNvdbUpperTable + 8 * (size_t)n);
+    return nullptr;
+  }
+  const unsigned char *lw = up + nvdb_ld<long long>(up + kNvdbUpperTable + 8 * (size_t)n);
+  n = (((uint32_t)x & 127u) >> 3 << 8) | (((uint32_t)y & 127u) >> 3 << 4) | (((uint32_t)z & 127u) >> 3);
+  if (!((nvdb_ld<uint64_t>(lw + kNvdbLowerChildMask + 8 * (n >> 6)) >> (n & 63)) & 1ull)) {
+    value = nvdb_ld<float>(lw + kNvdbLowerTable + 8 * (size_t)n);
+    return nullptr;
+  }
+  return lw + nvdb_ld<long long>(lw + kNvdbLowerTable + 8 * (size_t)n);
+}
+
 // ReadAccessor::getValue: the value at index coordinates (x, y, z) --
-// an active or inactive voxel, a tile value, or the background.
+// an active or inactive voxel, a tile value, or the background.  (Its own
+// walk: returning through nvdb_leaf cost NanoVDB frames 9%.)
 GBV_HD float nvdb_value(const NvdbGrid &g, int x, int y, int z) {
   const unsigned char *root = g.base + g.root;
   const uint64_t key = (uint64_t)((uint32_t)z >> 12) | ((uint64_t)((uint32_t)y >> 12) << 21) |

@@ -26,27 +26,77 @@ NvdbGrid make_nvdb_grid(const void *d_grid, const gbv_nanovdb_info &info) {
   return g;
 }
 
-// One thread per macrocell (NanoVDBData_computeMCs, NanoVDB.cu:28-60).
-__global__ void __launch_bounds__(128) nvdb_mc_ranges_kernel(NvdbGrid g, int ncx, int ncy, int ncz,
+// NanoVDBData_computeMCs (NanoVDB.cu:28-60), one block per macrocell.  The
+// macrocells of gbv_nanovdb_parse cover at most 18^3 voxels, which touch at
+// most 4^3 leaves: the block first walks the tree once per leaf (64 walks in
+// parallel), then its threads read the voxels straight from the leaves, z
+// fastest as a leaf stores them.  Larger macrocells (a caller's own mc_dims)
+// walk the tree at each voxel.  min and max are exact, so the order does not
+// matter.
+// What bounds it: the reads of the leaves (each voxel 1.4 times).  One thread
+// per macrocell walked the tree for each of its 5832 voxels, one after the
+// other: 2185 us for a 192^3 Float grid (1728 threads); this takes 32 us.
+constexpr int kNvdbMcLeaves = 4;
+constexpr int kNvdbMcThreads = 352;  // 18 x 18 columns in one go
+__global__ void __launch_bounds__(kNvdbMcThreads) nvdb_mc_ranges_kernel(NvdbGrid g, int ncx, int ncy, int ncz,
                                                              float2 *__restrict__ ranges) {
-  const long long n = (long long)ncx * ncy * ncz;
-  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (tid >= n) return;
-  int m[3] = {(int)(tid % ncx), (int)((tid / ncx) % ncy), (int)(tid / ((long long)ncx * ncy))};
-  const int mc[3] = {ncx, ncy, ncz};
+  __shared__ const unsigned char *s_leaf[kNvdbMcLeaves * kNvdbMcLeaves * kNvdbMcLeaves];
+  __shared__ float s_value[kNvdbMcLeaves * kNvdbMcLeaves * kNvdbMcLeaves];
+  __shared__ float2 s_part[kNvdbMcThreads / 32];
+  const long long mc = blockIdx.x;
+  int m[3] = {(int)(mc % ncx), (int)((mc / ncx) % ncy), (int)(mc / ((long long)ncx * ncy))};
+  const int count[3] = {ncx, ncy, ncz};
   const int size[3] = {g.hi[0] - g.lo[0] + 1, g.hi[1] - g.lo[1] + 1, g.hi[2] - g.lo[2] + 1};
   int a[3], b[3];
-  nvdb_mc_footprint(g.lo, size, mc, m, a, b);
+  nvdb_mc_footprint(g.lo, size, count, m, a, b);
+  // the leaves' 8^3 blocks the footprint touches
+  const int l0[3] = {a[0] >> 3, a[1] >> 3, a[2] >> 3};
+  const int n[3] = {(b[0] >> 3) - l0[0] + 1, (b[1] >> 3) - l0[1] + 1, (b[2] >> 3) - l0[2] + 1};
+  const bool staged = n[0] <= kNvdbMcLeaves && n[1] <= kNvdbMcLeaves && n[2] <= kNvdbMcLeaves;
+  for (int k = threadIdx.x; staged && k < n[0] * n[1] * n[2]; k += blockDim.x) {
+    const int z = k % n[2], y = (k / n[2]) % n[1], x = k / (n[2] * n[1]);
+    s_leaf[k] = nvdb_leaf(g, (l0[0] + x) << 3, (l0[1] + y) << 3, (l0[2] + z) << 3, s_value[k]);
+  }
+  __syncthreads();
   // range1f starts empty (+inf, -inf) and extends by min/max
   float lo = __int_as_float(0x7f800000), hi = __int_as_float(0xff800000);
-  for (int x = a[0]; x <= b[0]; x++)
-    for (int y = a[1]; y <= b[1]; y++)
-      for (int z = a[2]; z <= b[2]; z++) {
-        const float v = nvdb_value(g, x, y, z);
-        lo = mn(lo, v);
-        hi = mx(hi, v);
-      }
-  ranges[tid] = make_float2(lo, hi);
+  const int ey = b[1] - a[1] + 1, ez = b[2] - a[2] + 1;
+  const long long total = (long long)(b[0] - a[0] + 1) * ey * ez;
+  for (long long k = threadIdx.x; !staged && k < total; k += blockDim.x) {
+    const long long r = k / ez;
+    const float v = nvdb_value(g, a[0] + (int)(r / ey), a[1] + (int)(r % ey), a[2] + (int)(k % ez));
+    lo = mn(lo, v);
+    hi = mx(hi, v);
+  }
+  // a thread per (y, z) column: the divisions are once a column, and a leaf's
+  // rows of 8 values are read by 8 neighbouring threads
+  for (int k = threadIdx.x; staged && k < ey * ez; k += blockDim.x) {
+    const int z = a[2] + k % ez, y = a[1] + k / ez;
+    const int column = ((y >> 3) - l0[1]) * n[2] + (z >> 3) - l0[2];
+    const uint32_t in_leaf = ((uint32_t)(y & 7) << 3) | (uint32_t)(z & 7);
+#pragma unroll 6
+    for (int x = a[0]; x <= b[0]; x++) {
+      const int leaf = ((x >> 3) - l0[0]) * n[1] * n[2] + column;
+      const unsigned char *lf = s_leaf[leaf];
+      const float v = lf ? nvdb_leaf_value(g.type, lf, ((uint32_t)(x & 7) << 6) | in_leaf) : s_value[leaf];
+      lo = mn(lo, v);
+      hi = mx(hi, v);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = mn(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = mx(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = make_float2(lo, hi);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
+      lo = mn(lo, s_part[w].x);
+      hi = mx(hi, s_part[w].y);
+    }
+    ranges[mc] = make_float2(lo, hi);
+  }
 }
 
 __global__ void __launch_bounds__(128) nvdb_sample_kernel(NvdbGrid g, const float *__restrict__ P, long long n,
@@ -167,7 +217,7 @@ extern "C" gbv_status gbv_nanovdb_mc_ranges(const void *d_grid, const gbv_nanovd
   const NvdbGrid g = make_nvdb_grid(d_grid, *info);
   const long long n = (long long)info->mc_dims[0] * info->mc_dims[1] * info->mc_dims[2];
   if (n > (1ll << 31) - 1) return set_error(GBV_ERROR_UNSUPPORTED, "gbv_nanovdb_mc_ranges: too many macrocells");
-  nvdb_mc_ranges_kernel<<<(unsigned)((n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(
+  nvdb_mc_ranges_kernel<<<(unsigned)n, kNvdbMcThreads, 0, (cudaStream_t)stream>>>(
       g, info->mc_dims[0], info->mc_dims[1], info->mc_dims[2], reinterpret_cast<float2 *>(d_ranges));
   return check_launch("nvdb_mc_ranges_kernel");
 }
