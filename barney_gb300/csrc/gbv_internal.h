@@ -11,6 +11,10 @@ gbv_status set_error(gbv_status st, const char *msg);
 gbv_status check_launch(const char *what);
 gbv_status check_cuda(cudaError_t e, const char *what);
 
+// Scalar ranges of M macrocells of cpm cells a side (api.cu).
+gbv_status launch_mc_ranges(const float *d_scalars, const int dims[3], int cpm, const int M[3], float2 *ranges,
+                            cudaStream_t stream);
+
 // Stream-ordered scratch of a launch from the library's pool of the current
 // device (scratch.cpp); returned with cudaFreeAsync.
 cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);

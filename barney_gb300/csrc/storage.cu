@@ -5,9 +5,6 @@
 
 namespace gbv {
 
-__global__ void mc_ranges_kernel(const float *__restrict__ scalars, int nx, int ny, int nz, int cpm, int mx_,
-                                 int my_, int mz_, float2 *__restrict__ ranges);
-
 // One thread per cell of the padded brick grid, in store order, so each
 // thread writes one contiguous 8-voxel record.  Bricks have 2^lx x 2^ly x
 // 2^lz cells; U8 quantizes with the (min, max) of the cell's 8^3 scale brick
@@ -285,9 +282,7 @@ gbv_status gbv_build_brick_store_shaped(const float *d_scalars, const int dims[3
       break;
     case GBV_VOXEL_U8_SCALED: {
       // scale brick (min,max) over 9^3 voxels = the 8-cell macrocell range
-      mc_ranges_kernel<<<(unsigned)((scaleBricks + 7) / 8), 256, 0, cs>>>(d_scalars, dims[0], dims[1], dims[2], 8,
-                                                                          ns[0], ns[1], ns[2], lohi);
-      gbv_status st = check_launch("brick ranges");
+      gbv_status st = launch_mc_ranges(d_scalars, dims, 8, ns, lohi, cs);
       if (st != GBV_OK) return st;
       brick_store_kernel<GBV_VOXEL_U8_SCALED><<<blocks, 256, 0, cs>>>(d_scalars, GBV_STORE_ARGS, lohi, d_voxels);
       st = check_launch("brick_store_kernel");
