@@ -151,36 +151,48 @@ __device__ __forceinline__ StoreBrickCorners<FMT, true> via_l1(const StoreBrickC
 }
 
 // StructuredDataSampler::DD::sample (StructuredData.h:104-115) with the CPU
-// backend's trilinear filter (rtcore/embree/Texture.cpp:339-411).  NaN
-// outside [0, numCells).
-template <class Store>
-__device__ __forceinline__ float sample_field(const FieldGeom &F, const Store &S, vec3 P) {
-  vec3 rel = (P - F.origin) * F.rcpSpacing;
-  if (rel.x < 0.f || rel.y < 0.f || rel.z < 0.f) return __int_as_float(0x7fffffff);
-  if (rel.x >= (float)F.C[0] || rel.y >= (float)F.C[1] || rel.z >= (float)F.C[2])
-    return __int_as_float(0x7fffffff);
-  const vec3 tc = rel + vec3(.5f);
+// backend's trilinear filter (rtcore/embree/Texture.cpp:339-411), in two
+// parts: the stencil of a position (false outside [0, numCells)), and the
+// value at it.
+struct Stencil {
   int x0, x1, y0, y1, z0, z1;
   float fx, fy, fz;
-  lerp_coords(F.N[0], tc.x, x0, x1, fx);
-  lerp_coords(F.N[1], tc.y, y0, y1, fy);
-  lerp_coords(F.N[2], tc.z, z0, z1, fz);
+};
+__device__ __forceinline__ bool locate(const FieldGeom &F, vec3 P, vec3 &rel, Stencil &c) {
+  rel = (P - F.origin) * F.rcpSpacing;
+  if (rel.x < 0.f || rel.y < 0.f || rel.z < 0.f) return false;
+  if (rel.x >= (float)F.C[0] || rel.y >= (float)F.C[1] || rel.z >= (float)F.C[2]) return false;
+  const vec3 tc = rel + vec3(.5f);
+  lerp_coords(F.N[0], tc.x, c.x0, c.x1, c.fx);
+  lerp_coords(F.N[1], tc.y, c.y0, c.y1, c.fy);
+  lerp_coords(F.N[2], tc.z, c.z0, c.z1, c.fz);
+  return true;
+}
+template <class Store> __device__ __forceinline__ float value_at(const Store &S, Stencil s) {
   float c[8];
   if constexpr (Store::kCellStore) {
     // A clamped axis (x0 == x1) reads the same voxel twice with weight 0 on
     // the second; on a cell store that is cell 0 with f=0 or cell N-2 with
     // f=1, which gives the identical value for finite data.
-    if (x0 == x1) { if (x0 > 0) { x0 -= 1; fx = 1.f; } }
-    if (y0 == y1) { if (y0 > 0) { y0 -= 1; fy = 1.f; } }
-    if (z0 == z1) { if (z0 > 0) { z0 -= 1; fz = 1.f; } }
-    S.cell(x0, y0, z0, c);
+    if (s.x0 == s.x1) { if (s.x0 > 0) { s.x0 -= 1; s.fx = 1.f; } }
+    if (s.y0 == s.y1) { if (s.y0 > 0) { s.y0 -= 1; s.fy = 1.f; } }
+    if (s.z0 == s.z1) { if (s.z0 > 0) { s.z0 -= 1; s.fz = 1.f; } }
+    S.cell(s.x0, s.y0, s.z0, c);
   } else {
-    S.corners(x0, x1, y0, y1, z0, z1, c);
+    S.corners(s.x0, s.x1, s.y0, s.y1, s.z0, s.z1, c);
   }
-  const float v00 = lerp_l(fx, c[0], c[1]), v01 = lerp_l(fx, c[2], c[3]);
-  const float v10 = lerp_l(fx, c[4], c[5]), v11 = lerp_l(fx, c[6], c[7]);
-  const float v0 = lerp_l(fy, v00, v01), v1 = lerp_l(fy, v10, v11);
-  return lerp_l(fz, v0, v1);
+  const float v00 = lerp_l(s.fx, c[0], c[1]), v01 = lerp_l(s.fx, c[2], c[3]);
+  const float v10 = lerp_l(s.fx, c[4], c[5]), v11 = lerp_l(s.fx, c[6], c[7]);
+  const float v0 = lerp_l(s.fy, v00, v01), v1 = lerp_l(s.fy, v10, v11);
+  return lerp_l(s.fz, v0, v1);
+}
+// NaN outside [0, numCells)
+template <class Store>
+__device__ __forceinline__ float sample_field(const FieldGeom &F, const Store &S, vec3 P) {
+  vec3 rel;
+  Stencil c;
+  if (!locate(F, P, rel, c)) return __int_as_float(0x7fffffff);
+  return value_at(S, c);
 }
 
 // -------------------------------------------------------------------------

@@ -297,3 +297,82 @@ def test_differentiable_workload_at_its_named_size(cuda):
         fd = np.array([fd_of(lambda x, e=e: p.with_tf_entry(int(e), x), float(tfb[e])) for e in ent])
         an = gtf[ent]
         assert np.linalg.norm(fd - an) <= 1e-3 * np.linalg.norm(fd), (fd, an)
+
+
+def _march_both_ways(scene, views, step, store=None):
+    """The march in one call, whose pixels call for the search of empty
+    blocks, and view by view, which takes every step."""
+    import torch
+    both = EAProblem(scene, views, step, store=store).render()
+    each = torch.cat([EAProblem(scene, [v], step, store=store).render() for v in views])
+    torch.cuda.synchronize()
+    return both.cpu().numpy(), each.cpu().numpy()
+
+
+@pytest.mark.parametrize("dims", [(49, 49, 49), (65, 50, 57), (100, 64, 81)])
+@pytest.mark.parametrize("fmt", [None, N.GBV_VOXEL_F32, N.GBV_VOXEL_F16, N.GBV_VOXEL_U8_SCALED])
+@pytest.mark.parametrize("kind", ["two_peaks", "opaque", "nan_voxels", "inside", "far", "negative"])
+def test_skipped_steps_change_nothing(cuda, dims, fmt, kind):
+    """Empty space is skipped from 768 k pixels on: the image is the one that
+    takes every step, bit for bit, at block edges (a last block of one cell, a
+    clipped one), for rays along the faces, from inside the box and from far
+    away, with voxels that are NaN, with no empty block at all, and with
+    negative opacities."""
+    from barney_gb300.device import GpuScene
+    s = scenes.Scene(scalars=scenes.blob_volume(dims, 12, seed=8, noise=0.0), tf=scenes.tf_two_peaks(256),
+                     base_density=20.0)
+    views = scenes.fibonacci_views(4, 2.5, 8)
+    if kind == "opaque":
+        s.tf = scenes.tf_ramp(64) + np.float32(0.01)
+    if kind == "nan_voxels":
+        s.scalars[3, 5, 7] = np.nan
+    if kind == "negative":
+        s.tf[:, 3] *= -0.1
+    for k, v in enumerate(views):
+        v["width"], v["height"] = 640, 400
+        if kind == "inside":
+            v["pos"] = (0.1 * k, -0.05, 0.02)
+        if kind == "far":
+            v["pos"] = tuple(40.0 * x for x in v["pos"])
+            v["fovy"] = 1.0
+    views[0]["pos"], views[0]["dir"] = (0.0, 0.0, 2.0), (0.0, 0.0, -1.0)  # rays along the axes
+    store = GpuScene(s, fmt=fmt) if fmt is not None else None
+    both, each = _march_both_ways(s, views, 0.5 / (max(dims) - 1), store)
+    np.testing.assert_array_equal(both.view(np.uint32), each.view(np.uint32))
+
+
+@pytest.mark.parametrize("entry", [np.inf, np.nan, 1e38])
+def test_transfer_functions_that_rule_skipping_out(cuda, entry):
+    """An entry whose product with zero, or whose optical depth, is not finite."""
+    s = scenes.Scene(scalars=scenes.blob_volume((64, 64, 64), 12, seed=8, noise=0.0), tf=scenes.tf_two_peaks(256),
+                     base_density=20.0)
+    s.tf[10, 3 if entry == 1e38 else 0] = entry
+    views = scenes.fibonacci_views(4, 2.5, 8)
+    for v in views:
+        v["width"], v["height"] = 640, 400
+    both, each = _march_both_ways(s, views, 0.5 / 63)
+    np.testing.assert_array_equal(both.view(np.uint32), each.view(np.uint32))
+
+
+@pytest.mark.parametrize("w,h,nviews", [(1, 1, 1), (9, 5, 3), (33, 17, 2), (16, 8, 33)])
+def test_adjoint_tiles_of_uneven_views(cuda, w, h, nviews):
+    """Views whose tiles are partial, and more of them than one launch holds:
+    the gradients are the sums of the views' own (to the order of their
+    additions: each entry's rounding is below the sum of its terms' sizes
+    times the number of additions)."""
+    gt = scenes.ea_scene(24)
+    views = scenes.fibonacci_views(nviews, 2.5, 8)
+    for k, v in enumerate(views):
+        v["width"], v["height"] = w + k % 2, h
+    step = 0.5 / 23
+    p = EAProblem(gt, views, step)
+    img = p.render()
+    gv, gt_tf = p.backward(img, img)
+    sv, st, at = 0.0, 0.0, 0
+    for v in views:
+        n = v["width"] * v["height"]
+        part = img[at:at + n].contiguous()
+        a, b = EAProblem(gt, [v], step).backward(part, part)
+        sv, st, at = sv + a.double(), st + b.double(), at + n
+    np.testing.assert_allclose(gv.double().cpu(), sv.cpu(), rtol=1e-4, atol=1e-5 * float(sv.abs().max()))
+    np.testing.assert_allclose(gt_tf.double().cpu(), st.cpu(), rtol=1e-4, atol=1e-5 * float(st.abs().max()))
