@@ -65,6 +65,7 @@ struct EAParams {
   int eb[3];                 // blocks per axis
   int numViews;
   EAViewDev views[kMaxViewsPerLaunch];
+  int tileStart[kMaxViewsPerLaunch + 1];  // prefix sums of the views' 8x4-pixel tiles (the adjoint's work items)
 };
 
 template <typename R> struct V3T { R x, y, z; };
@@ -353,11 +354,14 @@ __global__ void __launch_bounds__(128) ea_forward_f64_kernel(const EAParams p, d
   out[v.offset + (long long)iy * v.W + ix] = res;
 }
 
-// Warp-aggregated flush of 8 per-corner (or per-TF-entry) gradient sums.
+// Warp-aggregated flush of 8 transfer-function gradient sums (two entries).
 // Lanes that flush in the same step and hold the same key are grouped with
 // __match_any_sync; the group's lowest lane gathers the others' sums by
 // shuffles and issues the 8 atomics once.  Called by all 32 lanes.
 // off(k) gives the destination index of sum k (evaluated by the leader only).
+// (Neighbouring rays often share a segment, and shared-memory atomics of one
+// address run one after the other: without grouping the adjoint is 5% slower.
+// Stencils are rarely shared in one step; grouping them cost 5%.)
 template <class Off>
 __device__ __forceinline__ void flush8(float *__restrict__ dst, bool flush, unsigned long long key, Off off,
                                        const float v[8]) {
@@ -390,159 +394,179 @@ __device__ __forceinline__ void flush8(float *__restrict__ dst, bool flush, unsi
 
 // FP32 adjoint by path replay.  Consecutive steps of a ray mostly stay in
 // the same cell and TF segment, so each lane keeps running sums for its
-// current stencil and TF segment and flushes them (warp-aggregated) only
-// when either changes.  Lanes run in lockstep up to the warp's longest march
-// (one extra iteration without steps flushes the last sums) so the flushes
-// see all 32 lanes.
+// current stencil and TF segment and adds them to the gradients only when a
+// step contributes to another one (steps on a flat stretch of the transfer
+// function contribute to no voxel).  Lanes run in lockstep up to the warp's
+// longest march (one extra iteration without steps flushes the last sums) so
+// the grouped flushes see all 32 lanes.
+//
+// The grid is as many blocks as fit; warps take 8x4-pixel tiles of the views
+// from a counter, and a block's transfer-function gradient stays in shared
+// memory until it is done.  A block per 16x8 pixels waited at its end for its
+// longest ray (1.25 of 8.6 stall cycles) and cleared and flushed the gradient
+// for every patch: 32 views of 256^2 through 128^3, 2168 us; this takes 1910.
 template <int MinBlocks>
 __global__ void __launch_bounds__(128, MinBlocks) ea_backward_kernel(const EAParams p, const float4 *__restrict__ img,
                                                           const float4 *__restrict__ gimg, float *__restrict__ gvox,
-                                                          float *__restrict__ gtf) {
+                                                          float *__restrict__ gtf, int *__restrict__ counter) {
   extern __shared__ float s_gtf[];  // tf_n*4, block-private TF gradient
   const int ntf = 4 * p.xf.n;
   for (int i = threadIdx.x; i < ntf; i += blockDim.x) s_gtf[i] = 0.f;
   __syncthreads();
-  const EAViewDev &v = p.views[blockIdx.z];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ix = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
-  const int iy = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
-  const bool inside = ix < v.W && iy < v.H;
-  vec3 org(0.f), dir(0.f, 0.f, 1.f);
-  float t0 = 0.f, t1 = 0.f;
-  int n = 0;
-  float4 C = make_float4(0.f, 0.f, 0.f, 0.f), g = C;
-  if (inside) {
-    const long long pix = v.offset + (long long)iy * v.W + ix;
-    if (ea_ray(p, v, ix, iy, org, dir, t0, t1, n)) {
-      C = img[pix];
-      g = gimg[pix];
-    } else {
-      n = 0;
-    }
-  }
-  const int nMax = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(n, 0));
-  const float Tn = 1.f - C.w;
-  const float gs = (float)(p.xf.n - 1) / p.xf.span;
-  const size_t sy = (size_t)p.F.N[0], sz = (size_t)p.F.N[0] * p.F.N[1];
-  const float bd = p.xf.baseDensity;
-  float A0 = 0.f, A1 = 0.f, A2 = 0.f;
-  // transmittance before the current step; the replay advances it as
-  // T_{i+1} = T_i - T_i alpha_i (alpha from expm1, so 1-alpha keeps full
-  // absolute precision): one transcendental per step
-  float T = 1.f;
-  bool alive = inside && n > 0;
-  // running sums: voxel stencil (key = 8 * base voxel + which axes are not
-  // clamped) and TF segment (key = idx)
-  long long vKey = -1;
-  float vAcc[8];
-  int tIdx = -1;
-  float tAcc[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) { vAcc[k] = 0.f; tAcc[k] = 0.f; }
-  for (int i = 0; i <= nMax; i++) {
-    // this step's contributions (none past the end of the lane's march)
-    bool have = false;
-    long long key = -1;
-    int idx = -1;
-    float fx = 0.f, fy = 0.f, fz = 0.f, dLds = 0.f, f = 0.f, dr = 0.f, dg = 0.f, db = 0.f, dsb = 0.f;
-    if (alive && i < n) {
-      const float t = t0 + ((float)i + .5f) * p.dt;
-      if (t >= t1) {
-        alive = false;
+  const int lane = threadIdx.x & 31;
+  while (true) {
+    int tile = 0;
+    if (lane == 0) tile = atomicAdd(counter, 1);
+    tile = __shfl_sync(0xffffffffu, tile, 0);
+    if (tile >= p.tileStart[p.numViews]) break;
+    int view = 0;
+    while (tile >= p.tileStart[view + 1]) view++;
+    tile -= p.tileStart[view];
+    const EAViewDev &v = p.views[view];
+    const int tilesX = (v.W + 7) >> 3;
+    const int ix = (tile % tilesX) * 8 + (lane & 7), iy = (tile / tilesX) * 4 + (lane >> 3);
+    const bool inside = ix < v.W && iy < v.H;
+    vec3 org(0.f), dir(0.f, 0.f, 1.f);
+    float t0 = 0.f, t1 = 0.f;
+    int n = 0;
+    float4 C = make_float4(0.f, 0.f, 0.f, 0.f), g = C;
+    if (inside) {
+      const long long pix = v.offset + (long long)iy * v.W + ix;
+      if (ea_ray(p, v, ix, iy, org, dir, t0, t1, n)) {
+        C = img[pix];
+        g = gimg[pix];
       } else {
-        const vec3 P = org + t * dir;
-        vec3 rel = (P - p.F.origin) * p.F.rcpSpacing;
-        const bool in = !(rel.x < 0.f || rel.y < 0.f || rel.z < 0.f || rel.x >= (float)p.F.C[0] ||
-                          rel.y >= (float)p.F.C[1] || rel.z >= (float)p.F.C[2]);
-        if (in) {
-          const vec3 tc = rel + vec3(.5f);
-          int x0, x1, y0, y1, z0, z1;
-          lerp_coords(p.F.N[0], tc.x, x0, x1, fx);
-          lerp_coords(p.F.N[1], tc.y, y0, y1, fy);
-          lerp_coords(p.F.N[2], tc.z, z0, z1, fz);
-          float c[8];
-          p.store.corners(x0, x1, y0, y1, z0, z1, c);
-          const float v00 = lerp_l(fx, c[0], c[1]), v01 = lerp_l(fx, c[2], c[3]);
-          const float v10 = lerp_l(fx, c[4], c[5]), v11 = lerp_l(fx, c[6], c[7]);
-          const float sv = lerp_l(fz, lerp_l(fy, v00, v01), lerp_l(fy, v10, v11));
-          f = (sv - p.xf.lo) / p.xf.span;
-          const bool clamped = !(f > 0.f && f < 1.f);
-          f = clampv(f, 0.f, 1.f);
-          f *= (float)(p.xf.n - 1);
-          idx = clampv((int)f, 0, p.xf.n - 2);
-          f -= (float)idx;
-          const float4 e0 = __ldg(p.xf.v + idx), e1 = __ldg(p.xf.v + idx + 1);
-          const float r = (1.f - f) * e0.x + f * e1.x, gg = (1.f - f) * e0.y + f * e1.y,
-                      b = (1.f - f) * e0.z + f * e1.z;
-          const float sig = ((1.f - f) * e0.w + f * e1.w) * bd;
-          const float x = sig * p.dt;
-          const float w = T * -expm1f(-x);
-          A0 += w * r;
-          A1 += w * gg;
-          A2 += w * b;
-          const float Tnext = T - w;
-          float dLdx = g.w * Tn;
-          dLdx += g.x * (r * Tnext - (C.x - A0));
-          dLdx += g.y * (gg * Tnext - (C.y - A1));
-          dLdx += g.z * (b * Tnext - (C.z - A2));
-          T = Tnext;
-          const float dLdsig = dLdx * p.dt;
-          dr = g.x * w;
-          dg = g.y * w;
-          db = g.z * w;
-          dsb = dLdsig * bd;
-          if (!clamped) {
-            dLds = dLdsig * bd * (e1.w - e0.w) * gs;
-            dLds += dr * (e1.x - e0.x) * gs + dg * (e1.y - e0.y) * gs + db * (e1.z - e0.z) * gs;
-            const size_t base = (size_t)x0 + sy * y0 + sz * z0;
-            key = 8 * (long long)base + (x1 != x0 ? 1 : 0) + (y1 != y0 ? 2 : 0) + (z1 != z0 ? 4 : 0);
-            have = true;
+        n = 0;
+      }
+    }
+    const int nMax = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(n, 0));
+    const float Tn = 1.f - C.w;
+    const float gs = (float)(p.xf.n - 1) / p.xf.span;
+    const size_t sy = (size_t)p.F.N[0], sz = (size_t)p.F.N[0] * p.F.N[1];
+    const float bd = p.xf.baseDensity;
+    float A0 = 0.f, A1 = 0.f, A2 = 0.f;
+    // transmittance before the current step; the replay advances it as
+    // T_{i+1} = T_i - T_i alpha_i (alpha from expm1, so 1-alpha keeps full
+    // absolute precision): one transcendental per step
+    float T = 1.f;
+    bool alive = inside && n > 0;
+    // running sums: voxel stencil (key = 8 * base voxel + which axes are not
+    // clamped) and TF segment (key = idx)
+    long long vKey = -1;
+    float vAcc[8];
+    int tIdx = -1;
+    float tAcc[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) { vAcc[k] = 0.f; tAcc[k] = 0.f; }
+    for (int i = 0; i <= nMax; i++) {
+      // this step's contributions (none past the end of the lane's march)
+      bool have = false;
+      long long key = -1;
+      int idx = -1;
+      float fx = 0.f, fy = 0.f, fz = 0.f, dLds = 0.f, f = 0.f, dr = 0.f, dg = 0.f, db = 0.f, dsb = 0.f;
+      if (alive && i < n) {
+        const float t = t0 + ((float)i + .5f) * p.dt;
+        if (t >= t1) {
+          alive = false;
+        } else {
+          const vec3 P = org + t * dir;
+          vec3 rel = (P - p.F.origin) * p.F.rcpSpacing;
+          const bool in = !(rel.x < 0.f || rel.y < 0.f || rel.z < 0.f || rel.x >= (float)p.F.C[0] ||
+                            rel.y >= (float)p.F.C[1] || rel.z >= (float)p.F.C[2]);
+          if (in) {
+            const vec3 tc = rel + vec3(.5f);
+            int x0, x1, y0, y1, z0, z1;
+            lerp_coords(p.F.N[0], tc.x, x0, x1, fx);
+            lerp_coords(p.F.N[1], tc.y, y0, y1, fy);
+            lerp_coords(p.F.N[2], tc.z, z0, z1, fz);
+            float c[8];
+            p.store.corners(x0, x1, y0, y1, z0, z1, c);
+            const float v00 = lerp_l(fx, c[0], c[1]), v01 = lerp_l(fx, c[2], c[3]);
+            const float v10 = lerp_l(fx, c[4], c[5]), v11 = lerp_l(fx, c[6], c[7]);
+            const float sv = lerp_l(fz, lerp_l(fy, v00, v01), lerp_l(fy, v10, v11));
+            f = (sv - p.xf.lo) / p.xf.span;
+            const bool clamped = !(f > 0.f && f < 1.f);
+            f = clampv(f, 0.f, 1.f);
+            f *= (float)(p.xf.n - 1);
+            idx = clampv((int)f, 0, p.xf.n - 2);
+            f -= (float)idx;
+            const float4 e0 = __ldg(p.xf.v + idx), e1 = __ldg(p.xf.v + idx + 1);
+            const float r = (1.f - f) * e0.x + f * e1.x, gg = (1.f - f) * e0.y + f * e1.y,
+                        b = (1.f - f) * e0.z + f * e1.z;
+            const float sig = ((1.f - f) * e0.w + f * e1.w) * bd;
+            const float x = sig * p.dt;
+            const float w = x == 0.f ? 0.f : T * -expm1f(-x);  // T is finite
+            A0 += w * r;
+            A1 += w * gg;
+            A2 += w * b;
+            const float Tnext = T - w;
+            float dLdx = g.w * Tn;
+            dLdx += g.x * (r * Tnext - (C.x - A0));
+            dLdx += g.y * (gg * Tnext - (C.y - A1));
+            dLdx += g.z * (b * Tnext - (C.z - A2));
+            T = Tnext;
+            const float dLdsig = dLdx * p.dt;
+            dr = g.x * w;
+            dg = g.y * w;
+            db = g.z * w;
+            dsb = dLdsig * bd;
+            if (!clamped) {
+              dLds = dLdsig * bd * (e1.w - e0.w) * gs;
+              dLds += dr * (e1.x - e0.x) * gs + dg * (e1.y - e0.y) * gs + db * (e1.z - e0.z) * gs;
+              // (a zero adds nothing: a flat stretch of the transfer function
+              // leaves the sums and their stencil alone)
+              have = dLds != 0.f;
+              const size_t base = (size_t)x0 + sy * y0 + sz * z0;
+              key = 8 * (long long)base + (x1 != x0 ? 1 : 0) + (y1 != y0 ? 2 : 0) + (z1 != z0 ? 4 : 0);
+            }
           }
         }
       }
-    }
-    // voxel stencil: flush the running sums when the stencil changes
-    const bool vFlush = vKey >= 0 && (key != vKey);
-    flush8(gvox, vFlush, (unsigned long long)vKey,
-           [&](int k) {
-             const size_t base = (size_t)(vKey >> 3);
-             const int m = (int)(vKey & 7) & k;
-             return base + ((m & 1) ? 1 : 0) + ((m & 2) ? sy : 0) + ((m & 4) ? sz : 0);
-           },
-           vAcc);
-    if (vFlush || vKey < 0) {
-      vKey = have ? key : -1;
+      // voxel stencil: flush the running sums when a step adds to another
+      // stencil, and after the last step
+      const bool vFlush = vKey >= 0 && ((have && key != vKey) || i == nMax);
+      if (vFlush) {
+        const size_t base = (size_t)(vKey >> 3);
 #pragma unroll
-      for (int k = 0; k < 8; k++) vAcc[k] = 0.f;
-    }
-    if (have) {
-      const float wx0 = 1.f - fx, wy0 = 1.f - fy, wz0 = 1.f - fz;
-      vAcc[0] += dLds * wx0 * wy0 * wz0;
-      vAcc[1] += dLds * fx * wy0 * wz0;
-      vAcc[2] += dLds * wx0 * fy * wz0;
-      vAcc[3] += dLds * fx * fy * wz0;
-      vAcc[4] += dLds * wx0 * wy0 * fz;
-      vAcc[5] += dLds * fx * wy0 * fz;
-      vAcc[6] += dLds * wx0 * fy * fz;
-      vAcc[7] += dLds * fx * fy * fz;
-    }
-    // TF segment: same scheme, into the block's shared-memory gradient
-    const bool tFlush = tIdx >= 0 && idx != tIdx;
-    flush8(s_gtf, tFlush, (unsigned long long)tIdx, [&](int k) { return 4 * tIdx + k; }, tAcc);
-    if (tFlush || tIdx < 0) {
-      tIdx = idx;
+        for (int k = 0; k < 8; k++) {
+          const int m = (int)(vKey & 7) & k;
+          if (vAcc[k] != 0.f) atomicAdd(gvox + base + ((m & 1) ? 1 : 0) + ((m & 2) ? sy : 0) + ((m & 4) ? sz : 0), vAcc[k]);
+        }
+      }
+      if (vFlush || vKey < 0) {
+        vKey = have ? key : -1;
 #pragma unroll
-      for (int k = 0; k < 8; k++) tAcc[k] = 0.f;
-    }
-    if (idx >= 0) {
-      tAcc[0] += dr * (1.f - f);
-      tAcc[1] += dg * (1.f - f);
-      tAcc[2] += db * (1.f - f);
-      tAcc[3] += dsb * (1.f - f);
-      tAcc[4] += dr * f;
-      tAcc[5] += dg * f;
-      tAcc[6] += db * f;
-      tAcc[7] += dsb * f;
+        for (int k = 0; k < 8; k++) vAcc[k] = 0.f;
+      }
+      if (have) {
+        const float wx0 = 1.f - fx, wy0 = 1.f - fy, wz0 = 1.f - fz;
+        vAcc[0] += dLds * wx0 * wy0 * wz0;
+        vAcc[1] += dLds * fx * wy0 * wz0;
+        vAcc[2] += dLds * wx0 * fy * wz0;
+        vAcc[3] += dLds * fx * fy * wz0;
+        vAcc[4] += dLds * wx0 * wy0 * fz;
+        vAcc[5] += dLds * fx * wy0 * fz;
+        vAcc[6] += dLds * wx0 * fy * fz;
+        vAcc[7] += dLds * fx * fy * fz;
+      }
+      // TF segment: same scheme, into the block's shared-memory gradient
+      const bool tFlush = tIdx >= 0 && idx != tIdx;
+      flush8(s_gtf, tFlush, (unsigned long long)tIdx, [&](int k) { return 4 * tIdx + k; }, tAcc);
+      if (tFlush || tIdx < 0) {
+        tIdx = idx;
+#pragma unroll
+        for (int k = 0; k < 8; k++) tAcc[k] = 0.f;
+      }
+      if (idx >= 0) {
+        tAcc[0] += dr * (1.f - f);
+        tAcc[1] += dg * (1.f - f);
+        tAcc[2] += db * (1.f - f);
+        tAcc[3] += dsb * (1.f - f);
+        tAcc[4] += dr * f;
+        tAcc[5] += dg * f;
+        tAcc[6] += db * f;
+        tAcc[7] += dsb * f;
+      }
     }
   }
   __syncthreads();
@@ -673,6 +697,10 @@ static gbv_status for_view_chunks(EAParams &p, const gbv_ea_view *views, int num
       d.W = v.width;
       d.H = v.height;
       d.offset = offset;
+      p.tileStart[k] = k ? p.tileStart[k] : 0;
+      const long long tiles = p.tileStart[k] + (((long long)v.width + 7) >> 3) * (((long long)v.height + 3) >> 2);
+      if (tiles > (1ll << 30)) return set_error(GBV_ERROR_INVALID_ARGUMENT, "ea: more than 2^30 tiles of 8x4 pixels");
+      p.tileStart[k + 1] = (int)tiles;
       offset += (long long)v.width * v.height;
       maxW = max(maxW, v.width);
       maxH = max(maxH, v.height);
@@ -749,16 +777,30 @@ gbv_status gbv_ea_backward_ex(const gbv_scene *s, const gbv_ea_view *views, int 
   // resident 128-thread blocks per SM the adjoint's registers are capped
   // for (default 6: 80 registers, no spills)
   const int occ = blocks_per_sm ? blocks_per_sm : 6;
-  return for_view_chunks(p, views, num_views, [&](EAParams &q, int cnt, int maxW, int maxH) {
-    dim3 grid((maxW + 15) / 16, (maxH + 7) / 8, cnt);
-    const float4 *img = reinterpret_cast<const float4 *>(d_images);
-    const float4 *gimg = reinterpret_cast<const float4 *>(d_grad_images);
-    cudaStream_t cs = (cudaStream_t)stream;
-    if (occ == 8) ea_backward_kernel<8><<<grid, 128, smem, cs>>>(q, img, gimg, d_grad_scalars, d_grad_tf);
-    else if (occ == 6) ea_backward_kernel<6><<<grid, 128, smem, cs>>>(q, img, gimg, d_grad_scalars, d_grad_tf);
-    else ea_backward_kernel<4><<<grid, 128, smem, cs>>>(q, img, gimg, d_grad_scalars, d_grad_tf);
-    return check_launch("ea_backward_kernel");
-  });
+  int dev = 0, sms = 0;
+  st = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+  if (st == GBV_OK) st = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+  // a tile counter per launch
+  const int launches = (num_views + kMaxViewsPerLaunch - 1) / kMaxViewsPerLaunch;
+  int *counters = nullptr;
+  cudaStream_t cs = (cudaStream_t)stream;
+  if (st == GBV_OK) st = check_cuda(scratch_alloc((void **)&counters, sizeof(int) * launches, cs), "gbv_ea_backward: scratch");
+  if (st != GBV_OK) return st;
+  st = check_cuda(cudaMemsetAsync(counters, 0, sizeof(int) * launches, cs), "gbv_ea_backward: scratch");
+  int launch = 0;
+  if (st == GBV_OK)
+    st = for_view_chunks(p, views, num_views, [&](EAParams &q, int cnt, int, int) {
+      const int tiles = q.tileStart[cnt], grid = std::min(sms * occ, (tiles + 3) / 4);
+      const float4 *img = reinterpret_cast<const float4 *>(d_images);
+      const float4 *gimg = reinterpret_cast<const float4 *>(d_grad_images);
+      int *counter = counters + launch++;
+      if (occ == 8) ea_backward_kernel<8><<<grid, 128, smem, cs>>>(q, img, gimg, d_grad_scalars, d_grad_tf, counter);
+      else if (occ == 6) ea_backward_kernel<6><<<grid, 128, smem, cs>>>(q, img, gimg, d_grad_scalars, d_grad_tf, counter);
+      else ea_backward_kernel<4><<<grid, 128, smem, cs>>>(q, img, gimg, d_grad_scalars, d_grad_tf, counter);
+      return check_launch("ea_backward_kernel");
+    });
+  const gbv_status fst = check_cuda(cudaFreeAsync(counters, cs), "gbv_ea_backward: scratch");
+  return st != GBV_OK ? st : fst;
 }
 
 gbv_status gbv_ea_backward(const gbv_scene *s, const gbv_ea_view *views, int num_views, float step,
