@@ -483,9 +483,9 @@ extern "C" gbv_status gbv_batch_create(const gbv_scene *scenes, float *const *d_
   b->hits = hits;
   if (st == GBV_OK) {
     // the log of split tiles: room for kBatchLogPasses passes of every tile,
-    // at most kLogBytes (more passes split fewer tiles); without it none are
+    // at most kBatchLogBytes (more passes split fewer tiles); without it none are
     const size_t want = (size_t)b->innerTiles * 32 * log_words(hits) * sizeof(uint32_t) * kBatchLogPasses;
-    b->logBytes = want < kLogBytes ? want : kLogBytes;
+    b->logBytes = want < kBatchLogBytes ? want : kBatchLogBytes;
     if (cudaMalloc((void **)&b->d_log, b->logBytes) != cudaSuccess) {
       cudaGetLastError();
       b->d_log = nullptr;

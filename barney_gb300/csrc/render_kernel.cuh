@@ -12,7 +12,7 @@
 // queued rays.
 #pragma once
 #include <cstring>
-#include <mutex>
+#include <type_traits>
 #include <vector>
 #include <cuda_runtime.h>
 #include "gbv_volume.cuh"
@@ -2086,8 +2086,11 @@ inline int path_hits(const RenderParams &p) {
   if (!p.multi || !p.volMS) return 1;
   return p.maxVB < 0 ? 1 : p.maxVB < 10 ? p.maxVB + 1 : 11;
 }
-// Log memory of a launch at most
-constexpr size_t kLogBytes = (size_t)256 << 20;
+// Log memory of a launch (of a batch) at most.  512^3, 1080p, 64 passes: not
+// in parts, a log for a tenth of the inner tiles 40.5 ms; in parts with 256 MB
+// 32.7 ms (31.0 with the 96-register budget), 512 MB 32.4 (30.5), 1 GB 31.5
+// (29.5), 3 GB 31.1 (29.2).
+constexpr size_t kLogBytes = (size_t)512 << 20, kBatchLogBytes = (size_t)256 << 20;
 constexpr int kBatchLogPasses = 16;
 // The rectangle of warp tiles the field's bounds project to (p.rx, ...);
 // returns the number of tiles in it.  A tile outside it provably sees nothing
@@ -2146,6 +2149,18 @@ inline long long plan_rect(RenderParams &p) {
     p.rw = p.rh = 1;
   }
   return (long long)p.rw * p.rh;
+}
+
+// Passes a launch renders at most: a frame of more passes than the log holds
+// for all of its inner tiles is rendered in parts that it does hold, as long as
+// a part has kPartPasses passes or more (the frame continues from the
+// accumulation buffer as progressive frames do).
+constexpr int kPartPasses = 4;
+inline int part_passes(const RenderParams &p, long long inner, int hits) {
+  const long long most = (long long)(kLogBytes / ((size_t)inner * 32 * log_words(hits) * sizeof(uint32_t)));
+  if (p.depth || p.primId || p.instId || p.objId || most < kPartPasses || p.spp <= most) return p.spp;
+  const long long parts = (p.spp + most - 1) / most;
+  return (int)((p.spp + parts - 1) / parts);
 }
 
 // What a launch over `inner` + `outer` tiles splits: as many of the last
@@ -2225,48 +2240,55 @@ inline gbv_status launch_render_t(const RenderParams &p, const Store &store, cud
   const size_t smem = p.isoOn ? plan_pool<true>(q, staged_words(p)) : plan_pool<false>(q, staged_words(p));
   long long blocks = 0;
   gbv_status st = GBV_OK;
-  // the tile pool counter and the majorant bitmask live in stream-ordered
-  // scratch memory (the mask at a 256-byte offset: 16-byte aligned for the
-  // bulk copy)
+  // the tile pool counter, the majorant bitmask and the log live in
+  // stream-ordered scratch memory (the mask at a 256-byte offset: 16-byte
+  // aligned for the bulk copy)
   int *pool = nullptr;
   const long long inner = plan_rect(q), outer = warp_tile_count(p) - inner;
-  size_t logBytes = plan_split(q, inner, outer, path_hits(p), kLogBytes);
+  const int hits = path_hits(p), most = part_passes(p, inner, hits);
+  q.spp = most;
+  size_t logBytes = plan_split(q, inner, outer, hits, kLogBytes);
   const size_t maskBytes = ((size_t)p.maskWords * 4 + 255) & ~(size_t)255;
   if (logBytes && scratch_alloc((void **)&pool, 256 + maskBytes + logBytes, stream) != cudaSuccess) {
     cudaGetLastError();  // no room for the log: no tile is split
-    logBytes = plan_split(q, inner, outer, 1, 0);
+    logBytes = 0;
   }
   if (!logBytes) st = check_cuda(scratch_alloc((void **)&pool, 256 + maskBytes, stream), "tile pool scratch");
   if (st != GBV_OK) return st;
-  if (logBytes) q.log = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(pool) + 256 + maskBytes);
-  st = plan_grid(q, kernel, smem, launch_tiles(q), blocks);
-  st = check_cuda(cudaMemsetAsync(pool, 0, sizeof(int), stream), "render_kernel: clearing the tile pool");
-  if (st == GBV_OK && p.maskWords > 0 && p.maskSrc == nullptr && p.maskMode == 0) {
+  if (p.maskWords > 0 && p.maskSrc == nullptr && p.maskMode == 0) {
     uint32_t *mask = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(pool) + 256);
     const int nmc = p.G.M[0] * p.G.M[1] * p.G.M[2];
     majorant_mask_kernel<<<(unsigned)((p.maskWords + 7) / 8), 256, 0, stream>>>(p.G.maj, nmc, p.maskWords, mask);
     st = check_launch("majorant_mask_kernel");
     q.maskSrc = mask;
   }
-  if (st == GBV_OK) {
-    kernel<<<(unsigned)blocks, block_threads(Budget), smem, stream>>>(q, nullptr, nullptr, 0, pool);
-    st = check_launch("render_kernel");
-  }
-  if (st == GBV_OK && q.log) {
-    resolve_kernel<false><<<(unsigned)((q.split * 32 + 255) / 256), 256, 0, stream>>>(q, nullptr, nullptr, 0);
-    st = check_launch("resolve_kernel");
+  const int step = logBytes ? most : p.spp;
+  for (int done = 0; st == GBV_OK && done < p.spp; done += step) {
+    q.accumIdStart = p.accumIdStart + done;
+    q.spp = p.spp - done < step ? p.spp - done : step;
+    if (plan_split(q, inner, outer, logBytes ? hits : 1, logBytes ? kLogBytes : 0))
+      q.log = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(pool) + 256 + maskBytes);
+    st = plan_grid(q, kernel, smem, launch_tiles(q), blocks);
+    if (st == GBV_OK)
+      st = check_cuda(cudaMemsetAsync(pool, 0, sizeof(int), stream), "render_kernel: clearing the tile pool");
+    if (st == GBV_OK) {
+      kernel<<<(unsigned)blocks, block_threads(Budget), smem, stream>>>(q, nullptr, nullptr, 0, pool);
+      st = check_launch("render_kernel");
+    }
+    if (st == GBV_OK && q.log) {
+      resolve_kernel<false><<<(unsigned)((q.split * 32 + 255) / 256), 256, 0, stream>>>(q, nullptr, nullptr, 0);
+      st = check_launch("resolve_kernel");
+    }
   }
   const gbv_status fst = check_cuda(cudaFreeAsync(pool, stream), "cudaFreeAsync(tile pool)");
   return st != GBV_OK ? st : fst;
 }
 
 // Launch settings resolved from a gbv_render_config (gbv_render_ex): the
-// resident 288-thread blocks per SM the registers are capped for (4: 36
-// warps per SM at 56 registers; 5 blocks give 45 warps at 40 registers and
-// spill more), and the shared-memory staging mode.  The traversal settings
+// register budget and the shared-memory staging mode.  The traversal settings
 // (skip, threshold) and the profile switch travel in RenderParams.
 struct LaunchChoice {
-  int occ = 4;
+  int occ = 0;  // 0: default_budget
   int stage = GBV_STAGE_DEFAULT;
   int mode = GBV_RENDER_PERSISTENT;
 };
@@ -2313,12 +2335,26 @@ inline void plan_staging(RenderParams &p, int stage) {
   }
 }
 
+// The register budget of a launch that asks for none: 20 warps of 96
+// registers for frames long enough to be bound by their middle (kManyPaths or
+// more paths that may see the field: 512^3 1080p 64 passes 32.4 -> 30.5 ms,
+// U8 1080p 32 passes 3.98 -> 3.73; 256^3 2560x1440 4 passes 3.77 -> 3.71), 16
+// of 128 for shorter ones, whose end waits for single paths (256^3 720p 1 pass
+// 0.50 ms, 0.60 with 20 warps; 853x479 8 passes 0.35, 0.40), for NanoVDB grids
+// (8.8 ms, 9.5) and iso-surfaces.
+constexpr long long kManyPaths = 4ll << 20;
+template <class Store> inline int default_budget(RenderParams p) {
+  if (std::is_same<Store, StoreNanoVDB>::value || p.isoOn) return 4;
+  return plan_rect(p) * 32 * p.spp >= kManyPaths ? 5 : 4;
+}
+
 template <class Store>
 inline gbv_status launch_render(RenderParams p, const Store &store, cudaStream_t stream, const LaunchChoice &lc) {
   plan_staging(p, lc.stage);
   if (!p.counters) p.profile = 0;
-  if (lc.occ <= 4 || p.isoOn) return launch_render_t<Store, 4>(p, store, stream);
-  if (lc.occ >= 6) return launch_render_t<Store, 6>(p, store, stream);
+  const int budget = p.isoOn ? 4 : lc.occ ? lc.occ : default_budget<Store>(p);
+  if (budget <= 4) return launch_render_t<Store, 4>(p, store, stream);
+  if (budget >= 6) return launch_render_t<Store, 6>(p, store, stream);
   return launch_render_t<Store, 5>(p, store, stream);
 }
 

@@ -15,7 +15,7 @@ namespace gbv {
 namespace {
 
 constexpr int kMaxDevices = 64;
-constexpr unsigned long long kKeepBytes = 320ull << 20;
+constexpr unsigned long long kKeepBytes = 576ull << 20;
 std::mutex g_mutex;
 cudaMemPool_t g_pools[kMaxDevices];
 

@@ -565,6 +565,20 @@ def batch_timing(count=64, reps=3):
     return out
 
 
+def own_launches(call) -> int:
+    """Kernel launches of this library in one call (counted in an untimed call;
+    a profiler's first session may record nothing, hence two)."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    n = 0
+    for _ in range(2):
+        with profile(activities=[ProfilerActivity.CUDA, ProfilerActivity.CPU]) as prof:
+            call()
+            torch.cuda.synchronize()
+        n = sum(1 for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA and "gbv::" in e.name)
+    return n
+
+
 def run_ours(args):
     import torch
     rank, world, local = dist_info()
@@ -638,9 +652,9 @@ def run_ours(args):
                          "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
                          else "fallback 6800 GB/s",
                          "bytes_per_launch": bytes_launch, "kernel": "render_kernel"},
-            # per frame: the majorant-bitmask kernel, then the render kernel
-            # (profiles/launches_bench_512cube_1080p_64spp.md)
-            "gpu_launches": 2 * args.steps, "clocks": clk.summary()}
+            # per frame: the majorant-bitmask kernel, then per part of the
+            # frame's passes the render kernel and the log's resolve kernel
+            "gpu_launches": own_launches(frame) * args.steps, "clocks": clk.summary()}
     # ---- e2e through the bn* C-ABI with host buffers, on every rank; the
     # slowest rank's step time counts ----
     if world > 1:

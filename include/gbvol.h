@@ -315,8 +315,8 @@ gbv_status gbv_render(const gbv_scene *scene, float *d_accum, int width,
    default, so a zero-initialised struct (or a null pointer) is the default
    launch.
    blocks_per_sm: the register budget, as resident 128-thread blocks per SM:
-     4 (default; 128 registers a thread), 5 or 6.  The persistent kernel runs
-     one block of that many threads on each SM.
+     4 (128 registers a thread), 5 or 6; by default 4, or 5 for long frames.
+     The persistent kernel runs one block of that many threads on each SM.
    threshold_pct: a warp keeps tracing while at least this percentage of its
      lanes is (1..100, default 25), or while no other stage has work for it.
    skip_cells: rounds (a cell test, a Woodcock distance draw and a step) a

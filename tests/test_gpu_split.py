@@ -38,17 +38,17 @@ def world(kind, w, h):
     away (the frame sees nothing of it) / tele (a pixel spans less than the
     rectangle's margin allows)."""
     s = scenes.small_scene(dims=40, spp=1, width=w, height=h)
-    if kind in ("multi", "forward", "iso"):
+    if kind in ("multi", "forward", "inside_forward", "iso"):
         s.multi_scatter = s.volume_multi_scatter = 1
         s.max_volume_bounces = 4
         s.env = scenes.env_sky(64, 32)
-    if kind == "forward":
+    if kind.endswith("forward"):
         s.anisotropy, s.max_volume_bounces = 0.8, 20
     if kind == "dark":
         s.bg_color = (0.5, 0.25, 0.125, -1.0)
     if kind == "iso":
         s.iso, s.volume_instance = scenes.IsoSurface(value=0.5), 1
-    if kind == "inside":
+    if kind.startswith("inside"):
         s.cam_pos = (0.05, 0.02, 0.03)
     if kind == "away":
         s.cam_dir = tuple(-x for x in s.cam_dir)
@@ -84,13 +84,16 @@ def test_split_frames_are_the_oracles(cuda, kind):
     np.testing.assert_array_equal(bits(a.cpu().numpy()), bits(oracle.Oracle(s).render(spp=4)))
 
 
-@pytest.mark.parametrize("kind,w,h,spp", [("inside", 640, 400, 72), ("forward", 320, 200, 40), ("inside", 200, 120, 2000)])
-def test_partly_split_equals_whole(cuda, kind, w, h, spp):
-    """The log has room for part of the inner tiles (the first two) or for so
-    few of them that none is split."""
+@pytest.mark.parametrize("kind,w,h,spp,start", [("inside", 640, 400, 220, 0), ("forward", 320, 200, 130, 3),
+                                                ("inside_forward", 1280, 800, 5, 0), ("inside", 200, 120, 2000, 0)])
+def test_frames_larger_than_the_log_equal_whole(cuda, kind, w, h, spp, start):
+    """Frames rendered in parts of as many passes as the log holds (the first
+    two, whose last parts are shorter), and one whose log does not hold enough
+    passes of all tiles, which splits part of them."""
     import torch
     g = GpuScene(world(kind, w, h))
-    a, b = g.render(spp=spp), whole(g, spp)
+    base = torch.rand(h, w, 4, device="cuda")
+    a, b = g.render(spp=spp, accum=base.clone(), accum_id_start=start), whole(g, spp, start, base.clone())
     torch.cuda.synchronize()
     np.testing.assert_array_equal(bits(a.cpu().numpy()), bits(b.cpu().numpy()))
 
