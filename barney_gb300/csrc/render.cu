@@ -339,19 +339,19 @@ extern "C" gbv_status gbv_tile_partition(int width, int height, int rank, int nu
 // render: an application that hands out all HBM from its own pre-sized pool
 // and requires libraries to work inside the buffers it passes them, or a
 // real-time viewer that forbids allocation and free calls on its frame
-// path (gbv_render takes its one scratch word from cudaMallocAsync and
+// path (gbv_render takes its scratch from cudaMallocAsync and
 // returns it with cudaFreeAsync, which draw on the device's memory pool).
-// This entry point takes that scratch word from a file-scope device array
+// This entry point takes its scratch, two words, from a file-scope device array
 // instead.
 // ===========================================================================
 namespace gbv {
 
-// The persistent kernel's only scratch: the tile-pool counter (one 32-bit
-// word).  Every GPU that loads this library holds this array until the
+// The only scratch: the tile counters of the frame kernel and of the kernel
+// that finishes the frame (two 32-bit words).  Every GPU that loads this library holds this array until the
 // process exits.  All calls share it and it keeps the last call's value, so
 // each call clears it first; calls that overlap on the GPU (for example on
 // two streams) race on it.
-static __device__ __align__(256) int g_noalloc_tile_pool[1];
+static __device__ __align__(256) int g_noalloc_tile_pool[2];
 constexpr long long kNoAllocMaxTiles = 1ll << 30;
 
 // Device address of the scratch on the current device.  Host code may not
@@ -479,7 +479,7 @@ extern "C" gbv_status gbv_batch_create(const gbv_scene *scenes, float *const *d_
   if (st == GBV_OK) st = check_cuda(cudaMalloc((void **)&b->d_items, sizeof(RenderParams) * count), "gbv_batch_create");
   if (st == GBV_OK)
     st = check_cuda(cudaMalloc((void **)&b->d_tileStart, sizeof(long long) * 2 * (count + 1)), "gbv_batch_create");
-  if (st == GBV_OK) st = check_cuda(cudaMalloc((void **)&b->d_pool, sizeof(int)), "gbv_batch_create");
+  if (st == GBV_OK) st = check_cuda(cudaMalloc((void **)&b->d_pool, 2 * sizeof(int)), "gbv_batch_create");
   b->hits = hits;
   if (st == GBV_OK) {
     // the log of split tiles: room for kBatchLogPasses passes of every tile,

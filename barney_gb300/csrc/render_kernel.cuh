@@ -66,11 +66,11 @@ struct RenderParams {
   int poolOff;    // the block's path pool starts here
   int slots;      // path slots a block uses (a multiple of 32)
   // The warp tiles that may see the field (its projection's rectangle, in
-  // tiles): handed out first, numbered row by row; the other tiles follow
+  // tiles), numbered row by row; the other tiles are the outer ones
   int rx, ry, rw, rh;
   // What the launch hands out: `whole` inner tiles with all their passes, then
   // each pass of `split` inner tiles by itself (its fragments logged and added
-  // up in order by resolve_kernel), then the outer tiles
+  // up in order by finish_kernel, which also renders the outer tiles)
   long long whole, split, outer;
   uint32_t *log;  // null: split == 0
   int logHits;    // fragments a record has room for
@@ -117,7 +117,7 @@ __host__ __device__ inline long long warp_tile_count(const RenderParams &p) {
 }
 
 // what one launch hands out (see RenderParams::whole)
-__host__ __device__ inline long long launch_tiles(const RenderParams &L) { return L.whole + L.split * L.spp + L.outer; }
+__host__ __device__ inline long long launch_tiles(const RenderParams &L) { return L.whole + L.split * L.spp; }
 // the i-th tile inside (outside) the field's rectangle, row-major
 __device__ __forceinline__ int inner_tile(const RenderParams &p, int i) {
   const int tilesX = (int)(((long long)p.W + 7) >> 3);
@@ -131,13 +131,16 @@ __device__ __forceinline__ int outer_tile(const RenderParams &p, int i) {
   const int col = i % side;
   return (p.ry + i / side) * tilesX + (col < p.rx ? col : col + p.rw);
 }
-// the last item whose first tile is at or before t
-__device__ __forceinline__ int tile_item(const long long *__restrict__ start, int numItems, long long t) {
-  int lo = 0, hi = numItems - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (start[mid] <= t) lo = mid;
-    else hi = mid - 1;
+// the last item whose first tile is at or before t, searched by the whole
+// warp: a load per 32-fold of items
+__device__ __forceinline__ int tile_item_warp(const long long *__restrict__ start, int numItems, long long t) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0, n = numItems;  // it is one of lo .. lo + n - 1
+  while (n > 1) {
+    const int step = (n + 31) / 32, i = lo + lane * step;
+    const int at = __popc(__ballot_sync(0xffffffffu, lane * step < n && start[i] <= t)) - 1;
+    n = min(step, n - at * step);
+    lo += at * step;
   }
   return lo;
 }
@@ -862,7 +865,7 @@ constexpr int kBatchSkipDefault = 64;
 constexpr int kThresholdDefault = 25;
 constexpr int kRefillMin = 12, kFull = 28;
 constexpr int kRepeatMin = 24;     // lanes for which starting passes goes on
-constexpr int kIdlePolls = 4096;   // polls (200 ns) of a warp without work
+constexpr int kIdlePolls = 1 << 24;  // polls (1 us) of a warp without work
 
 // Per-lane event counts; with On == false the counting and its registers
 // compile away (timed launches pass no counter buffer).
@@ -1287,6 +1290,26 @@ __device__ __forceinline__ void generate_primary(const RenderParams &p, int ix, 
   ray.numDiffuseBounces = 0;
 }
 
+// A primary ray that leaves the world: its fragment, and its alpha in w
+__device__ __forceinline__ float4 primary_miss(const RenderParams &p, int iy, vec3 dir, int accumID) {
+  const float4 miss = miss_color(p, iy);
+  vec3 frag(miss.x, miss.y, miss.z);
+  if (p.hasEnv) {
+    const float2 uv = env_miss_coords(p, dir);
+    const float4 t = tex2D(p.env, uv.x, uv.y);
+    frag = p.env.scale * vec3(t.x, t.y, t.z);
+  }
+  frag = vmin(frag, vec3(10.f * (float)(1 + accumID)));
+  return make_float4(frag.x, frag.y, frag.z, miss.w);
+}
+__device__ __forceinline__ void add_miss(float4 &acc, float4 miss, int accumID) {
+  if (accumID == 0) {
+    acc = miss;
+  } else {
+    if (miss.w > 0.f) acc.w += miss.w;
+    accum_add(acc, vec3(miss.x, miss.y, miss.z));
+  }
+}
 // What a path waits for; each is a bitmask over the block's slots in shared
 // memory.  Publishing a path sets its bit (after a fence), taking it clears
 // the bit: whoever clears it owns the path.
@@ -1301,7 +1324,7 @@ enum {
 // Control word of a path: flags, generation in bits 8..15
 constexpr uint32_t F_FRESH = 1u, F_SHADOW = 2u, F_ALIVE = 4u, F_ISOBOX = 8u, F_SPLIT = 16u,
                    F_LONE = 32u /* a shadow ray of a path that goes on elsewhere */,
-                   F_OUTER = 64u /* a pixel outside the field's rectangle */, F_VOLHIT = 1u << 16, F_SURFHIT = 2u << 16,
+                   F_VOLHIT = 1u << 16, F_SURFHIT = 2u << 16,
                    kHitMask = 3u << 16;
 // Words of a path's record.  The main ray's hit (t, rgb, the surface's
 // normal) shares the shadow ray's words: a main ray's hit is shaded before
@@ -1478,6 +1501,7 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
   const unsigned lt = (1u << lane) - 1u;
   const int rot = 2 * warp;
   const RenderParams &L = p0;  // launch-wide settings
+  asm volatile("griddepcontrol.launch_dependents;");  // finish_kernel may start where a block has ended
   // ---- stage the majorant bitmask and env-map tables in shared memory ----
   if (!Batch) {
     const RenderParams &p = p0;
@@ -1579,10 +1603,10 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
     else stage = nHit == most ? S_HIT : Iso && nIso == most ? S_ISO : S_START;
     if (stage == S_NONE) {
       // Nothing waits: the block is done, or its paths are with other warps.
-      // Those go on with what becomes of them, so a warp may leave; it looks
-      // again for a while to share what comes.
+      // What becomes of them may need this warp (it may hold a tile whose
+      // pixels wait for slots), so it looks again; each path ends, so does this.
       if ((poolDone && P.waiting(Q_FREE) == L.slots) || ++idle > kIdlePolls) break;
-      __nanosleep(200);
+      __nanosleep(idle < 64 ? 200 : 1000);
       continue;
     }
     idle = 0;
@@ -1641,8 +1665,14 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
         }
         if (cur >= 0) {
           const RenderParams &p = Batch ? items[P.u(W_ITEM, cur)] : p0;
-          if (T.inCell != 2 && trace_seek(p.G, T, cnt, L.skip, !Batch && L.maskWords > 0, L.capFlag) == TR_MISS)
-            ended = cur;
+          if (T.inCell != 2) {
+            if constexpr (Batch) {
+              const MCGridDev G = p.G;  // in registers while it seeks
+              if (trace_seek(G, T, cnt, L.skip, false, L.capFlag) == TR_MISS) ended = cur;
+            } else {
+              if (trace_seek(p.G, T, cnt, L.skip, L.maskWords > 0, L.capFlag) == TR_MISS) ended = cur;
+            }
+          }
           __syncwarp(act);  // the lanes with a position sample together
           if (T.inCell == 2) {
             Hit h;
@@ -1779,7 +1809,7 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
       phase = 0;
       int n;
       int k = nStart ? P.take(Q_START, 32, rot, n) : (n = 0, -1);
-      bool mine = k >= 0, fresh = false, outer = false;
+      bool mine = k >= 0, fresh = false;
       int ix = 0, iy = 0, s = 0, gen = 0, item = 0;
       uint32_t split = 0u, rec = 0u, mask = 0u;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1789,7 +1819,6 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
         const uint32_t ctl = P.u(W_CTL, k);
         fresh = ctl & F_FRESH;
         split = ctl & F_SPLIT;
-        outer = ctl & F_OUTER;
         ix = (int)P.u(W_IX, k);
         iy = (int)P.u(W_IY, k);
         s = (int)P.u(W_PASS, k);
@@ -1814,7 +1843,7 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
       uint32_t *const own = P.queue(Q_COUNT) + 1 + 6 * warp;
       int tile = (int)own[0], tileTaken = (int)own[1], tileItem = (int)own[2], tilePass = (int)own[3];
       uint32_t tileRec = own[4];  // log record of a split tile's first pixel
-      bool tileSplit = own[5] & 1u, tileOuter = own[5] & 2u;
+      bool tileSplit = own[5] & 1u;
       while (true) {
         // pixels for the lanes that hold a free slot
         while (true) {
@@ -1828,26 +1857,21 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
               poolDone = true;
               break;
             }
+            const long long j = t - L.whole;
             tileTaken = 0;
             tilePass = 0;
             long long idx = t;
-            const long long j = t - L.whole;
-            tileOuter = j >= L.split * L.spp;
-            tileSplit = j >= 0 && !tileOuter;
+            tileSplit = j >= 0;
             if (tileSplit) {
               tileRec = (uint32_t)j * 32u;
               tilePass = (int)((uint32_t)j % (uint32_t)L.spp);
               idx = L.whole + (uint32_t)j / (uint32_t)L.spp;
-            } else if (tileOuter) {
-              idx = j - L.split * L.spp;
             }
             if (Batch) {  // the item whose tiles idx falls in
-              const long long *start = tileOuter ? tileStart + numItems + 1 : tileStart;
-              tileItem = tile_item(start, numItems, idx);
-              idx -= start[tileItem];
+              tileItem = tile_item_warp(tileStart, numItems, idx);
+              idx -= tileStart[tileItem];
             }
-            const RenderParams &tp = Batch ? items[tileItem] : p0;
-            tile = tileOuter ? outer_tile(tp, (int)idx) : inner_tile(tp, (int)idx);
+            tile = inner_tile(Batch ? items[tileItem] : p0, (int)idx);
           }
           const RenderParams &tp = Batch ? items[tileItem] : p0;
           int tx, ty;
@@ -1862,7 +1886,6 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
               iy = py;
               s = tilePass;
               split = tileSplit ? F_SPLIT : 0u;
-              outer = tileOuter;
               rec = tileRec + (uint32_t)at;
               mask = 0u;
               acc = L.accumIdStart == 0 || tileSplit ? make_float4(0.f, 0.f, 0.f, 0.f)
@@ -1875,21 +1898,15 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
         const RenderParams &p = Batch ? items[item] : p0;
         bool missed = mine && !fresh;
         if (mine && fresh) {
-          // a pixel outside the rectangle sees nothing of the field: its ray
-          // matters to the env map alone
           PathRay ray;
-          bool enters = false;
           gen = 0;
-          if (!outer || p.hasEnv) generate_primary(p, ix, iy, L.accumIdStart + s, ray);
-          if (!outer) {
-            vec3 tdir = ray.dir;
-            if (tdir.x == 0.f) tdir.x = 1e-6f;
-            if (tdir.y == 0.f) tdir.y = 1e-6f;
-            if (tdir.z == 0.f) tdir.z = 1e-6f;
-            float tLo = 0.f, tHi = ray.tMax;
-            enters = box_test(ray.org, tdir, tLo, tHi, p.F.boundsLo, p.F.boundsHi);
-          }
-          if (enters) {
+          generate_primary(p, ix, iy, L.accumIdStart + s, ray);
+          vec3 tdir = ray.dir;
+          if (tdir.x == 0.f) tdir.x = 1e-6f;
+          if (tdir.y == 0.f) tdir.y = 1e-6f;
+          if (tdir.z == 0.f) tdir.z = 1e-6f;
+          float tLo = 0.f, tHi = ray.tMax;
+          if (box_test(ray.org, tdir, tLo, tHi, p.F.boundsLo, p.F.boundsHi)) {
             P.setv3(W_ORG, k, ray.org);
             P.setv3(W_DIR, k, ray.dir);
             P.setu64(W_SEED, k, ray.seed.state);
@@ -1919,35 +1936,28 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
           const int accumID = L.accumIdStart + s;
           if (!Batch && gen == 0 && (p.depth || p.primId || p.instId || p.objId))
             write_aux(p, (size_t)iy * p.W + ix, accumID, 1e30f, 0);
-          vec3 env(0.f);
-          if (p.hasEnv) {
-            const float2 uv = env_miss_coords(p, dir);
-            const float4 t = tex2D(p.env, uv.x, uv.y);
-            env = p.env.scale * vec3(t.x, t.y, t.z);
-          } else if (gen != 0) {
-            env = vec3(p.ambient);
-          }
-          const float4 miss = miss_color(p, iy);
           vec3 frag;
-          float alpha = 0.f;
+          float alpha = 1.f;
           if (gen == 0) {
-            alpha = miss.w;
-            frag = p.hasEnv ? env : vec3(miss.x, miss.y, miss.z);
+            const float4 m = primary_miss(p, iy, dir, accumID);
+            frag = vec3(m.x, m.y, m.z);
+            alpha = m.w;
           } else {
-            frag = weight * env * mis;
+            vec3 env(p.ambient);
+            if (p.hasEnv) {
+              const float2 uv = env_miss_coords(p, dir);
+              const float4 t = tex2D(p.env, uv.x, uv.y);
+              env = p.env.scale * vec3(t.x, t.y, t.z);
+            }
+            frag = vmin(weight * env * mis, vec3(10.f * (float)(1 + accumID)));
           }
-          frag = vmin(frag, vec3(10.f * (float)(1 + accumID)));
           if (split) {
             log_fragment(L, rec, gen, frag);
-            log_end(L, rec, mask | (1u << gen) | (gen == 0 ? kLogMissed : 0u), gen == 0 ? alpha : 1.f);
+            log_end(L, rec, mask | (1u << gen) | (gen == 0 ? kLogMissed : 0u), alpha);
             mine = false;
           } else {
-            if (accumID == 0 && gen == 0) {
-              acc = make_float4(frag.x, frag.y, frag.z, alpha);
-            } else {
-              if (gen == 0 && alpha > 0.f) acc.w += alpha;
-              accum_add(acc, frag);
-            }
+            if (gen == 0) add_miss(acc, make_float4(frag.x, frag.y, frag.z, alpha), accumID);
+            else accum_add(acc, frag);
             if (++s == L.spp) {
               p.accum[(size_t)iy * p.W + ix] = acc;
               mine = false;
@@ -1964,7 +1974,7 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
         own[2] = (uint32_t)tileItem;
         own[3] = (uint32_t)tilePass;
         own[4] = tileRec;
-        own[5] = (tileSplit ? 1u : 0u) | (tileOuter ? 2u : 0u);
+        own[5] = tileSplit ? 1u : 0u;
       }
       if (mine) {
         P.setacc(k, acc);
@@ -1972,7 +1982,7 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
         P.setu(W_IX, k, (uint32_t)ix);
         P.setu(W_IY, k, (uint32_t)iy);
         if (Batch) P.setu(W_ITEM, k, (uint32_t)item);
-        P.setu(W_CTL, k, F_FRESH | (outer ? F_OUTER : 0u));
+        P.setu(W_CTL, k, F_FRESH);
       }
       if (k >= 0) P.publish(mine ? Q_START : Q_FREE, k);
     } else {
@@ -2032,48 +2042,144 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
   }
 }
 
-// Adds up the logged fragments of the split tiles: one thread per pixel,
-// pass by pass and generation by generation.
+// A lane's pixel of a warp tile; false past the frame's edge
 template <bool Batch>
-static __global__ void __launch_bounds__(256) resolve_kernel(const __grid_constant__ RenderParams L,
-                                                             const RenderParams *__restrict__ items,
-                                                             const long long *__restrict__ tileStart, int numItems) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >> 5 >= L.split) return;
-  const long long t = L.whole + (i >> 5);
-  const int item = Batch ? tile_item(tileStart, numItems, t) : 0;
-  const RenderParams &p = Batch ? items[item] : L;
-  const int at = (int)(i & 31);
-  int tx, ty;
-  tile_corner<Batch>(L, p, inner_tile(p, (int)(Batch ? t - tileStart[item] : t)), tx, ty);
-  tx += at & 7;
-  ty += at >> 3;
-  if (tx >= p.W || ty >= p.H) return;
-  float4 *out = p.accum + (size_t)ty * p.W + tx;
-  float4 acc = L.accumIdStart == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *out;
-  const int words = log_words(L.logHits);
-  const uint32_t *r = L.log + ((size_t)(i >> 5) * L.spp * 32 + at) * words;
-  for (int s = 0; s < L.spp; s++, r += (size_t)32 * words) {
-    uint32_t mask = r[0];
-    const float alpha = __uint_as_float(r[1]);
-    const float *f = reinterpret_cast<const float *>(r + 2);
-    if (L.accumIdStart + s == 0) {
-      acc = make_float4(0.f, 0.f, 0.f, alpha);
-      if (mask & kLogMissed) {
-        acc.x = f[0];
-        acc.y = f[1];
-        acc.z = f[2];
-        continue;
+__device__ __forceinline__ bool tile_pixel(const RenderParams &L, const RenderParams &p, int tile, int lane, int &ix,
+                                           int &iy) {
+  tile_corner<Batch>(L, p, tile, ix, iy);
+  ix += lane & 7;
+  iy += lane >> 3;
+  return ix < p.W && iy < p.H;
+}
+// What the frame kernel leaves of a frame: the outer tiles, whose rays see
+// nothing of the field, and the sums of the split tiles' fragments.  A lane
+// per pixel, a warp per tile, passes in order.  It is launched with the frame
+// kernel (programmatic stream serialization): its blocks start on the SMs
+// that run out of paths first and fill them with the outer tiles (taken from
+// pool[1]) until the last path has ended; then they add up the log.
+//
+// As stages of the frame kernel the outer tiles took path slots, registers and
+// instruction cache from the rest: 64 scenes of 8 passes 5.52 -> 5.20 ms, 1080p
+// 512^3 of one pass 0.76 -> 0.70 ms without them there.  Taken one by one, the
+// counter they are taken from bounds them (64 scenes of one pass 0.79 ms, in
+// groups 0.73 ms).  The sums are bound by the log's reads, one round trip per
+// kAhead passes (64 scenes of 8 passes: 5.14 -> 5.12 ms, 256^2 of 16 passes 0.142
+// -> 0.138 ms from 4 passes at a time; 8 at a time the same).
+constexpr int kFinishThreads = 256;
+template <bool Batch>
+static __global__ void __launch_bounds__(kFinishThreads)
+    finish_kernel(const __grid_constant__ RenderParams L, const RenderParams *__restrict__ items,
+                  const long long *__restrict__ tileStart, int numItems, int *__restrict__ pool, int group) {
+  const int lane = threadIdx.x & 31;
+  while (L.outer > 0) {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(pool + 1, group);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t >= L.outer) break;
+    for (const int end = (int)min((long long)t + group, L.outer); t < end; t++) {
+      long long idx = t;
+      int item = 0;
+      if (Batch) {
+        item = tile_item_warp(tileStart + numItems + 1, numItems, idx);
+        idx -= tileStart[numItems + 1 + item];
       }
-    } else if (alpha > 0.f) {
-      acc.w += alpha;
-    }
-    for (mask &= ~kLogMissed; mask; mask &= mask - 1) {
-      const float *g = f + 3 * (__ffs(mask) - 1);
-      accum_add(acc, vec3(g[0], g[1], g[2]));
+      const RenderParams &p = Batch ? items[item] : L;
+      int ix, iy;
+      const bool inside = tile_pixel<Batch>(L, p, outer_tile(p, (int)idx), lane, ix, iy);
+      if (L.counters) {
+        const int rays = __popc(__ballot_sync(0xffffffffu, inside));
+        if (lane == 0) atomicAdd(L.counters + 2, (unsigned long long)rays * L.spp);
+      }
+      if (inside) {
+        const size_t at = (size_t)iy * p.W + ix;
+        float4 acc = L.accumIdStart == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : p.accum[at];
+        for (int s = 0; s < L.spp; s++) {
+          const int accumID = L.accumIdStart + s;
+          PathRay ray;
+          if (p.hasEnv) generate_primary(p, ix, iy, accumID, ray);
+          if (!Batch && (p.depth || p.primId || p.instId || p.objId)) write_aux(p, at, accumID, 1e30f, 0);
+          add_miss(acc, primary_miss(p, iy, ray.dir, accumID), accumID);
+        }
+        p.accum[at] = acc;
+      }
+      __syncwarp();
     }
   }
-  *out = acc;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the frame kernel is complete
+  const long long warps = (long long)gridDim.x * (kFinishThreads / 32);
+  for (long long k = ((long long)blockIdx.x * kFinishThreads + threadIdx.x) >> 5; k < L.split; k += warps) {
+    const long long t = L.whole + k;
+    const int item = Batch ? tile_item_warp(tileStart, numItems, t) : 0;
+    const RenderParams &p = Batch ? items[item] : L;
+    int ix, iy;
+    if (!tile_pixel<Batch>(L, p, inner_tile(p, (int)(Batch ? t - tileStart[item] : t)), lane, ix, iy)) continue;
+    float4 *out = p.accum + (size_t)iy * p.W + ix;
+    float4 acc = L.accumIdStart == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *out;
+    const int words = log_words(L.logHits);
+    const uint32_t *r = L.log + ((size_t)k * L.spp * 32 + lane) * words;
+    // kAhead records at a time, all their first words asked for at once (a
+    // path's first fragment is the only one of most records; where it logged
+    // none its words are not used)
+    constexpr int kAhead = 4;
+    for (int s0 = 0; s0 < L.spp; s0 += kAhead, r += (size_t)kAhead * 32 * words) {
+      uint32_t head[kAhead][5];
+#pragma unroll
+      for (int a = 0; a < kAhead; a++)
+#pragma unroll
+        for (int w = 0; w < 5; w++) head[a][w] = s0 + a < L.spp ? r[(size_t)a * 32 * words + w] : 0u;
+#pragma unroll
+      for (int a = 0; a < kAhead; a++) {
+        if (s0 + a >= L.spp) break;
+        uint32_t mask = head[a][0];
+        const float alpha = __uint_as_float(head[a][1]);
+        const vec3 first(__uint_as_float(head[a][2]), __uint_as_float(head[a][3]), __uint_as_float(head[a][4]));
+        if (L.accumIdStart + s0 + a == 0) {
+          acc = make_float4(0.f, 0.f, 0.f, alpha);
+          if (mask & kLogMissed) {
+            acc.x = first.x;
+            acc.y = first.y;
+            acc.z = first.z;
+            continue;
+          }
+        } else if (alpha > 0.f) {
+          acc.w += alpha;
+        }
+        if (mask & 1u) accum_add(acc, first);
+        for (mask &= ~(kLogMissed | 1u); mask; mask &= mask - 1) {
+          const float *g = reinterpret_cast<const float *>(r + (size_t)a * 32 * words + 2) + 3 * (__ffs(mask) - 1);
+          accum_add(acc, vec3(g[0], g[1], g[2]));
+        }
+      }
+    }
+    *out = acc;
+  }
+}
+// After the frame kernel of the same launch.
+template <bool Batch>
+inline gbv_status launch_finish(const RenderParams &L, const RenderParams *items, const long long *tileStart, int numItems,
+                                int *pool, cudaStream_t stream) {
+  if (L.outer + L.split == 0) return GBV_OK;
+  int dev = 0, sms = 0;
+  gbv_status st = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+  if (st == GBV_OK) st = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+  if (st != GBV_OK) return st;
+  const int warps = kFinishThreads / 32;
+  const long long tiles = L.outer > L.split ? L.outer : L.split, most = (long long)sms * 8;
+  const long long blocks = (tiles + warps - 1) / warps;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(blocks < most ? blocks : most));
+  cfg.blockDim = dim3(kFinishThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute serial;
+  serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  serial.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &serial;
+  cfg.numAttrs = 1;
+  // outer tiles a warp takes at a time: a few turns for each warp of the GPU
+  const long long turns = L.outer / (most * warps * 2);
+  const int group = (int)(turns < 1 ? 1 : turns > 16 ? 16 : turns);
+  return check_cuda(cudaLaunchKernelEx(&cfg, finish_kernel<Batch>, L, items, tileStart, numItems, pool, group),
+                    "finish_kernel");
 }
 
 // Fragments a path of this world can log: one per hit (its shadow ray) or
@@ -2211,7 +2317,7 @@ inline gbv_status plan_grid(RenderParams &p, RenderKernelFn kernel, size_t smem,
   if (st != GBV_OK) return st;
   blocks = tiles < sms ? tiles : sms;
   if (blocks < 1) blocks = 1;
-  const long long share = 32 * ((tiles + blocks - 1) / blocks);
+  const long long share = (p.split ? 64 : 32) * ((tiles + blocks - 1) / blocks);
   p.slots = (int)(share < kSlots ? share : kSlots);
   return GBV_OK;
 }
@@ -2270,15 +2376,12 @@ inline gbv_status launch_render_t(const RenderParams &p, const Store &store, cud
       q.log = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(pool) + 256 + maskBytes);
     st = plan_grid(q, kernel, smem, launch_tiles(q), blocks);
     if (st == GBV_OK)
-      st = check_cuda(cudaMemsetAsync(pool, 0, sizeof(int), stream), "render_kernel: clearing the tile pool");
+      st = check_cuda(cudaMemsetAsync(pool, 0, 2 * sizeof(int), stream), "render_kernel: clearing the tile pool");
     if (st == GBV_OK) {
       kernel<<<(unsigned)blocks, block_threads(Budget), smem, stream>>>(q, nullptr, nullptr, 0, pool);
       st = check_launch("render_kernel");
     }
-    if (st == GBV_OK && q.log) {
-      resolve_kernel<false><<<(unsigned)((q.split * 32 + 255) / 256), 256, 0, stream>>>(q, nullptr, nullptr, 0);
-      st = check_launch("resolve_kernel");
-    }
+    if (st == GBV_OK) st = launch_finish<false>(q, nullptr, nullptr, 0, pool, stream);
   }
   const gbv_status fst = check_cuda(cudaFreeAsync(pool, stream), "cudaFreeAsync(tile pool)");
   return st != GBV_OK ? st : fst;
@@ -2378,10 +2481,11 @@ inline gbv_status launch_render_noalloc(RenderParams p, const Store &store, cuda
   long long blocks = 0;
   gbv_status st = plan_grid(p, kernel, smem, launch_tiles(p), blocks);
   if (st != GBV_OK) return st;
-  st = check_cuda(cudaMemsetAsync(pool, 0, sizeof(int), stream), "gbv_render_noalloc: clearing the tile pool");
+  st = check_cuda(cudaMemsetAsync(pool, 0, 2 * sizeof(int), stream), "gbv_render_noalloc: clearing the tile pool");
   if (st != GBV_OK) return st;
   kernel<<<(unsigned)blocks, block_threads(4), smem, stream>>>(p, nullptr, nullptr, 0, pool);
-  return check_launch("render_kernel (noalloc)");
+  st = check_launch("render_kernel (noalloc)");
+  return st != GBV_OK ? st : launch_finish<false>(p, nullptr, nullptr, 0, pool, stream);
 }
 
 }  // namespace gbv
@@ -2408,17 +2512,16 @@ inline gbv_status batch_launch_t(const gbv_batch *b, RenderParams L, cudaStream_
                                            : render_kernel<Store, Budget, true, false>;
   const size_t smem = plan_pool<false>(L, 0);
   long long blocks = 0;
-  if (plan_split(L, b->innerTiles, b->outerTiles, b->hits, b->logBytes)) L.log = b->d_log;
+  // One pass each has no passes to split, and many scenes' pixels fill the GPU
+  // by themselves: 64 scenes 0.82 -> 0.80 ms without the log
+  const size_t room = L.spp > 1 ? b->logBytes : 0;
+  if (plan_split(L, b->innerTiles, b->outerTiles, b->hits, room)) L.log = b->d_log;
   gbv_status st = plan_grid(L, kernel, smem, launch_tiles(L), blocks);
-  if (st == GBV_OK) st = check_cuda(cudaMemsetAsync(b->d_pool, 0, sizeof(int), stream), "gbv_batch_render: pool");
+  if (st == GBV_OK) st = check_cuda(cudaMemsetAsync(b->d_pool, 0, 2 * sizeof(int), stream), "gbv_batch_render: pool");
   if (st != GBV_OK) return st;
   kernel<<<(unsigned)blocks, block_threads(Budget), smem, stream>>>(L, b->d_items, b->d_tileStart, b->count, b->d_pool);
   st = check_launch("render_kernel (batch)");
-  if (st == GBV_OK && L.log) {
-    resolve_kernel<true><<<(unsigned)((L.split * 32 + 255) / 256), 256, 0, stream>>>(L, b->d_items, b->d_tileStart,
-                                                                                     b->count);
-    st = check_launch("resolve_kernel (batch)");
-  }
+  if (st == GBV_OK) st = launch_finish<true>(L, b->d_items, b->d_tileStart, b->count, b->d_pool, stream);
   return st;
 }
 template <class Store>

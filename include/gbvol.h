@@ -402,15 +402,15 @@ gbv_status gbv_unpack_tiles(const void *d_tiles, int width, int height,
    allocate device memory while they render (an application that hands out
    all HBM from its own pre-sized pool, or a real-time viewer that forbids
    allocation calls on its frame path).  No counterpart in the reference.
-   Same arguments and results as gbv_render.  Its one word of scratch (the
-   persistent kernel's tile-pool counter) lives in a file-scope device array
-   of 4 bytes that every GPU loading this library keeps until exit, instead
+   Same arguments and results as gbv_render.  Its two words of scratch
+   (the kernels' tile counters) live in a file-scope device array of 8 bytes
+   that every GPU loading this library keeps until exit, instead
    of a cudaMallocAsync/cudaFreeAsync pair.  Every call looks up that
    array's device address on the current device (cudaGetSymbolAddress, which
    allocates nothing), so a device reset between calls is harmless; the first
    call on a device (or after a reset) may load the library's device code
-   there, so make it before any stream capture.  All calls share the word and each
-   call clears it before its launch, so calls that overlap on the GPU (for
+   there, so make it before any stream capture.  All calls share the words and each
+   call clears them before its launch, so calls that overlap on the GPU (for
    example on two streams) race.  Frames above 2^30 tiles of 8x4 pixels are
    rejected with GBV_ERROR_INVALID_ARGUMENT. */
 gbv_status gbv_render_noalloc(const gbv_scene *scene, float *d_accum, int width,

@@ -159,3 +159,21 @@ def test_captured_render_replays(cuda):
         graph.replay()
         torch.cuda.synchronize()
         np.testing.assert_array_equal(bits(acc.cpu().numpy()), bits(ref.cpu().numpy()))
+
+
+@pytest.mark.parametrize("kind", ["single", "dark", "multi"])
+def test_background_taken_in_groups_equals_wavefront(cuda, kind):
+    """A frame with more background tiles than the GPU has warps twice over
+    (they are taken several at a time), ragged at its right and lower edge,
+    alone and in a batch of two, against the wavefront mode."""
+    import torch
+    s = world(kind, 2043, 1301)
+    s.fovy = 120.0
+    g = GpuScene(s)
+    ref = g.render(spp=3, config={"mode": N.GBV_RENDER_WAVEFRONT})
+    acc = g.render(spp=3)
+    batch = GpuBatch([s, s])
+    batch.render(3)
+    torch.cuda.synchronize()
+    for a in [acc, whole(g, 3)] + list(batch.accums):
+        np.testing.assert_array_equal(bits(a.cpu().numpy()), bits(ref.cpu().numpy()))
