@@ -108,12 +108,12 @@ GBV_EA_BRICK_STORE(GBV_VOXEL_U8_SCALED)
 // the image is the same, bit for bit, when
 // * every transfer-function entry and the density are finite, so that 0 times
 //   a colour is 0, and the optical depth cannot become infinite (whose next
-//   compensation would be NaN), and the domain is positive (ea_skippable);
+//   compensation would be NaN), and the domain is positive (check_transfer);
 // * the block's range of stored values, widened by what the trilinear
 //   interpolation can round past it (7 lerps: below 16 ulp), covers only
 //   entries of zero opacity (empty_kernel); NaN samples have no opacity.
 // The next step to take is the first that may leave the block: the steps'
-// positions are bounded kEdge away from its faces, more than the positions
+// positions are bounded `edge` away from its faces, more than the positions
 // round (a few ulp of a cell index).
 //
 // The march is bound by its samples' loads (89% of the L1 throughput on the

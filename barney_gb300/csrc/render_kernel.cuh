@@ -1061,6 +1061,9 @@ __device__ __forceinline__ int trace_sample(const FieldGeom &F, const Store &sto
   return TR_CONTINUE;
 }
 
+// i / 10 as a float
+static __constant__ float kTenths[11] = {0.f / 10.f, 1.f / 10.f, 2.f / 10.f, 3.f / 10.f, 4.f / 10.f, 5.f / 10.f,
+                                         6.f / 10.f, 7.f / 10.f, 8.f / 10.f, 9.f / 10.f, 10.f / 10.f};
 // The hit search and normal of MCIsoSurfaceAccel::isProg
 // (MCAccelerator.h:393-503) along a DDA that trace_begin set up: per
 // macrocell whose scalar range holds the iso value, the cell's t range is
@@ -1082,38 +1085,50 @@ __device__ __forceinline__ bool iso_search(const FieldGeom &F, const Store &rend
   const int maxCells = G.M[0] + G.M[1] + G.M[2] + 8;
   float tHit = tmax;
   bool stopped = false;
+  auto crosses = [&](float tt0, float ff0, float tt1, float ff1) {
+    if (isnan(ff0) || isnan(ff1) || !(iso >= mn(ff0, ff1) && iso <= mx(ff0, ff1))) return false;
+    float t = (iso - ff0) / (ff1 - ff0);
+    t = lerp_l(t, tt0, tt1);
+    tHit = mn(tHit, t);
+    return tHit < tmax;
+  };
+  // Each lane walks to its next macrocell that holds the value, then all of
+  // them sample theirs: a cell's 11 samples are most of the search, and a lane
+  // that sampled where it stood left those that had only to walk on waiting
+  // (256^3, 960x540, 8 passes through isotropic fog: 5.78 -> 5.22 ms; two samples at a time 6.4,
+  // at most 8 cells a walk the same).
+  bool more = true;
 #pragma unroll 1
-  for (int it = 0; it < maxCells; it++) {
-    const float tc = reduce_min(T.t_next);
-    const float t0 = T.ray_t0 + T.ncb;
-    const float t1 = T.ray_t0 + mn(tc, T.tMax);
-    if (t0 > stop + fabsf(stop) * 1e-5f) break;
-    // the iso lambda (MCAccelerator.h:405-471)
-    if (!(t0 >= mn(t1, tmax))) {
-      const float2 vr = __ldg(ranges + (T.cx + G.M[0] * (T.cy + G.M[1] * T.cz)));
-      if (iso >= vr.x && iso <= vr.y) {
-        float tt1 = t0;
-        float ff1 = sample_field(F, store, T.org + tt1 * T.dir);
+  for (int it = 0; more;) {
+    float tc = 0.f, t0 = 0.f, t1 = 0.f;
+    bool holds = false;
 #pragma unroll 1
-        for (int i = 1; i <= 10; i++) {
-          const float tt0 = tt1;
-          const float ff0 = ff1;
-          tt1 = lerp_l((float)i / 10.f, t0, t1);
-          ff1 = sample_field(F, store, T.org + tt1 * T.dir);
-          if (isnan(ff0) || isnan(ff1)) continue;
-          if (iso >= mn(ff0, ff1) && iso <= mx(ff0, ff1)) {
-            float t = (iso - ff0) / (ff1 - ff0);
-            t = lerp_l(t, tt0, tt1);
-            tHit = mn(tHit, t);
-            if (tHit < tmax) {
-              stopped = true;
-              break;
-            }
-          }
-        }
+    while (more && !holds) {
+      more = it++ < maxCells;
+      tc = reduce_min(T.t_next);
+      t0 = T.ray_t0 + T.ncb;
+      t1 = T.ray_t0 + mn(tc, T.tMax);
+      more = more && !(t0 > stop + fabsf(stop) * 1e-5f);
+      if (!more) break;
+      // the iso lambda (MCAccelerator.h:405-471)
+      if (!(t0 >= mn(t1, tmax))) {
+        const float2 vr = __ldg(ranges + (T.cx + G.M[0] * (T.cy + G.M[1] * T.cz)));
+        holds = iso >= vr.x && iso <= vr.y;
       }
+      if (!holds) more = trace_advance(T, tc);
     }
-    if (stopped || !trace_advance(T, tc)) break;
+    if (!holds) break;
+    float tt1 = t0;
+    float ff1 = sample_field(F, store, T.org + tt1 * T.dir);
+#pragma unroll 1
+    for (int i = 1; i <= 10 && !stopped; i++) {
+      const float tt0 = tt1;
+      const float ff0 = ff1;
+      tt1 = lerp_l(kTenths[i], t0, t1);
+      ff1 = sample_field(F, store, T.org + tt1 * T.dir);
+      stopped = crosses(tt0, ff0, tt1, ff1);
+    }
+    more = !stopped && trace_advance(T, tc);
   }
   if (!(tHit < tmax)) return false;
   const vec3 P = T.org + tHit * T.dir;
