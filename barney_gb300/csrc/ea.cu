@@ -108,7 +108,9 @@ GBV_EA_BRICK_STORE(GBV_VOXEL_U8_SCALED)
 // the image is the same, bit for bit, when
 // * every transfer-function entry and the density are finite, so that 0 times
 //   a colour is 0, and the optical depth cannot become infinite (whose next
-//   compensation would be NaN), and the domain is positive (check_transfer);
+//   compensation would be NaN); no opacity is negative, so that the
+//   transmittance is at most 1 (negative ones can make it infinite, and 0 times
+//   that is NaN); and the domain is positive (check_transfer);
 // * the block's range of stored values, widened by what the trilinear
 //   interpolation can round past it (7 lerps: below 16 ulp), covers only
 //   entries of zero opacity (empty_kernel); NaN samples have no opacity.
@@ -131,13 +133,14 @@ __device__ __forceinline__ bool range_occupied(const XF &xf, float lo, float hi)
   return false;
 }
 // The transfer function's part of the conditions (the first block's threads):
-// finite entries, and an optical depth that stays finite over kEAMaxSteps.
+// finite entries, no negative opacity, and an optical depth that stays finite
+// over kEAMaxSteps.
 __device__ __forceinline__ void check_transfer(const XF &xf, float dt, EmptyBlocks *out) {
   bool bad = !(xf.span > 0.f) || !isfinite(xf.lo) || !isfinite(xf.span);
   for (int i = threadIdx.x; i < xf.n; i += blockDim.x) {
     const float4 e = __ldg(xf.v + i);
     bad = bad || !isfinite(e.x) || !isfinite(e.y) || !isfinite(e.z) ||
-          !(fabsf(e.w) * fabsf(xf.baseDensity) * dt * (float)kEAMaxSteps < 1e37f);
+          e.w * xf.baseDensity < 0.f || !(fabsf(e.w) * fabsf(xf.baseDensity) * dt * (float)kEAMaxSteps < 1e37f);
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) out->refused = 1;
 }

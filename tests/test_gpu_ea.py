@@ -354,6 +354,24 @@ def test_transfer_functions_that_rule_skipping_out(cuda, entry):
     np.testing.assert_array_equal(both.view(np.uint32), each.view(np.uint32))
 
 
+@pytest.mark.parametrize("fmt", [None, N.GBV_VOXEL_F16])
+def test_infinite_transmittance_is_not_skipped(cuda, fmt):
+    """Opacities so negative that the transmittance overflows: a step of zero
+    opacity past that point is 0 times infinity, in the march that looks for
+    empty blocks as in the one that takes every step."""
+    from barney_gb300.device import GpuScene
+    s = scenes.Scene(scalars=scenes.blob_volume((64, 64, 64), 12, seed=8, noise=0.0), tf=scenes.tf_two_peaks(256),
+                     base_density=20.0)
+    s.tf[:, 3] *= -40.0
+    views = scenes.fibonacci_views(4, 2.5, 8)
+    for v in views:
+        v["width"], v["height"] = 640, 400
+    store = GpuScene(s, fmt=fmt) if fmt is not None else None
+    both, each = _march_both_ways(s, views, 0.5 / 63, store)
+    assert np.isnan(each).any()
+    np.testing.assert_array_equal(both.view(np.uint32), each.view(np.uint32))
+
+
 @pytest.mark.parametrize("w,h,nviews", [(1, 1, 1), (9, 5, 3), (33, 17, 2), (16, 8, 33)])
 def test_adjoint_tiles_of_uneven_views(cuda, w, h, nviews):
     """Views whose tiles are partial, and more of them than one launch holds:
