@@ -498,7 +498,8 @@ __global__ void __launch_bounds__(128, MinBlocks) ea_backward_kernel(const EAPar
                         b = (1.f - f) * e0.z + f * e1.z;
             const float sig = ((1.f - f) * e0.w + f * e1.w) * bd;
             const float x = sig * p.dt;
-            const float w = x == 0.f ? 0.f : T * -expm1f(-x);  // T is finite
+            // alpha is x where x is 0 (negative opacities can have made T infinite)
+            const float w = T * (x == 0.f ? x : -expm1f(-x));
             A0 += w * r;
             A1 += w * gg;
             A2 += w * b;

@@ -372,6 +372,28 @@ def test_infinite_transmittance_is_not_skipped(cuda, fmt):
     np.testing.assert_array_equal(both.view(np.uint32), each.view(np.uint32))
 
 
+def test_adjoint_of_an_infinite_transmittance(cuda):
+    """A slab of opacity -40 (30 steps of depth -13: the transmittance is
+    infinite past it), then one of opacity 0: a step there has the weight
+    infinity times 0, and so have the gradients of its transfer-function
+    segment."""
+    import torch
+    n = 32
+    s = scenes.Scene(scalars=np.full((n, 8, 8), 0.75, np.float32),
+                     tf=np.ones((5, 4), np.float32), base_density=20.0)
+    s.scalars[n // 2:] = 0.25  # the camera's side: entry 1 of 0..4; the far side: entry 3
+    s.tf[:3, 3], s.tf[3:, 3] = -40.0, 0.0
+    view = dict(scenes.fibonacci_views(1, 2.5, 8)[0], width=1, height=1, pos=(0.0, 0.0, 2.0), dir=(0.0, 0.0, -1.0),
+                up=(0.0, 1.0, 0.0))
+    p = EAProblem(s, [view], 0.5 / (n - 1))
+    img = p.render()
+    gv, gt = p.backward(img, torch.ones_like(img))
+    torch.cuda.synchronize()
+    assert np.isnan(img.cpu().numpy()[0, :3]).all()
+    # the segment of entries 3 and 4 is met at opacity 0 alone
+    assert np.isnan(gt.cpu().numpy()[3:]).all()
+
+
 @pytest.mark.parametrize("w,h,nviews", [(1, 1, 1), (9, 5, 3), (33, 17, 2), (16, 8, 33)])
 def test_adjoint_tiles_of_uneven_views(cuda, w, h, nviews):
     """Views whose tiles are partial, and more of them than one launch holds:
