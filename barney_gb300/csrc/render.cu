@@ -2,6 +2,7 @@
 // (camera, lights, env map, macrocell grid) and dispatch to the kernels of
 // the scene's voxel store (render_store_*.cu).
 #include <cstdio>
+#include "gbvol_diag.h"
 #include "render_kernel.cuh"
 
 namespace gbv {
@@ -213,7 +214,8 @@ static bool resolve_config(const gbv_render_config *c, RenderParams &p, LaunchCh
 
 static gbv_status render_frame(const char *fn, const gbv_scene *s, float *d_accum, int width, int height,
                                int accum_id_start, int spp, int rank, int num_ranks, unsigned long long *d_counters,
-                               void *stream, int *d_cap_flag = nullptr, const gbv_render_config *config = nullptr) {
+                               void *stream, int *d_cap_flag = nullptr, const gbv_render_config *config = nullptr,
+                               int idle_polls = kIdlePolls) {
   char msg[160];
   if (!s || !d_accum || width <= 0 || height <= 0 || spp < 0 || accum_id_start < 0) {
     snprintf(msg, sizeof msg, "%s: null pointer or non-positive size", fn);
@@ -261,6 +263,7 @@ static gbv_status render_frame(const char *fn, const gbv_scene *s, float *d_accu
   p.spp = spp;
   p.counters = d_counters;
   p.capFlag = d_cap_flag;
+  p.idlePolls = idle_polls;
   p.rank = rank;
   p.numRanks = num_ranks;
   if (warp_tile_count(p) == 0) return GBV_OK;  // a rank that owns no tile
@@ -305,6 +308,14 @@ extern "C" gbv_status gbv_render_ex(const gbv_scene *s, float *d_accum, int widt
                                     void *stream) {
   return render_frame("gbv_render_ex", s, d_accum, width, height, accum_id_start, spp, 0, 1, d_counters, stream,
                       nullptr, config);
+}
+
+extern "C" gbv_status gbv_selftest_idle_limit(const gbv_scene *s, float *d_accum, int width, int height, int spp,
+                                              int idle_polls, unsigned long long *d_counters, int *d_cap_flag,
+                                              void *stream) {
+  if (idle_polls < 0) return set_error(GBV_ERROR_INVALID_ARGUMENT, "gbv_selftest_idle_limit: negative limit");
+  return render_frame("gbv_selftest_idle_limit", s, d_accum, width, height, 0, spp, 0, 1, d_counters, stream,
+                      d_cap_flag, nullptr, idle_polls);
 }
 
 extern "C" gbv_status gbv_render_tiles(const gbv_scene *s, float *d_accum, int width, int height,
@@ -527,6 +538,7 @@ extern "C" gbv_status gbv_batch_render(gbv_batch *b, int accum_id_start, int spp
   L.counters = d_counters;
   L.skip = b->skip;
   L.threshold = b->threshold;
+  L.idlePolls = kIdlePolls;
   L.maskWords = 0;
   L.cdfYOff = L.pivOff = L.rowOff = -1;
   L.profile = 0;

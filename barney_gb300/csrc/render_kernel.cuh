@@ -55,6 +55,7 @@ struct RenderParams {
   int *capFlag;   // if set, a loop-cap event stores 1 here (no counting needed)
   int skip;       // seek rounds per traversal iteration
   int threshold;  // keep tracing while at least this % of the lanes does
+  int idlePolls;  // a warp that finds no work this many times in a row gives up (a loop-cap event)
   // shared-memory staging (offsets in 32-bit words of the dynamic smem)
   int maskWords;  // >0: bitmask of non-zero majorants staged at offset 0 (a multiple of 4 words)
   const uint32_t *maskSrc;  // the bitmask in HBM (16-byte aligned), staged by one bulk copy; null: by ballots
@@ -865,7 +866,7 @@ constexpr int kBatchSkipDefault = 64;
 constexpr int kThresholdDefault = 25;
 constexpr int kRefillMin = 12, kFull = 28;
 constexpr int kRepeatMin = 24;     // lanes for which starting passes goes on
-constexpr int kIdlePolls = 1 << 24;  // polls (1 us) of a warp without work
+constexpr int kIdlePolls = 1 << 24;  // polls (1 us) a warp without work makes at most
 
 // Per-lane event counts; with On == false the counting and its registers
 // compile away (timed launches pass no counter buffer).
@@ -1638,7 +1639,14 @@ __global__ void __launch_bounds__(block_threads(Budget), 1)
       // Nothing waits: the block is done, or its paths are with other warps.
       // What becomes of them may need this warp (it may hold a tile whose
       // pixels wait for slots), so it looks again; each path ends, so does this.
-      if ((poolDone && P.waiting(Q_FREE) == L.slots) || ++idle > kIdlePolls) break;
+      if (poolDone && P.waiting(Q_FREE) == L.slots) break;
+      if (++idle > L.idlePolls) {  // pixels of its tile may be missing
+        if (lane == 0) {
+          GBV_COUNT(cnt, caps);
+          if (L.capFlag) *L.capFlag = 1;
+        }
+        break;
+      }
       __nanosleep(idle < 64 ? 200 : 1000);
       continue;
     }
@@ -2163,7 +2171,9 @@ static __global__ void __launch_bounds__(kFinishThreads)
 #pragma unroll
       for (int a = 0; a < kAhead; a++) {
         if (s0 + a >= L.spp) break;
-        uint32_t mask = head[a][0];
+        // (no bit past the record's fragments: a pass that a warp gave up on,
+        // see idlePolls, has logged nothing)
+        uint32_t mask = head[a][0] & (kLogMissed | ((1u << L.logHits) - 1u));
         const float alpha = __uint_as_float(head[a][1]);
         const vec3 first(__uint_as_float(head[a][2]), __uint_as_float(head[a][3]), __uint_as_float(head[a][4]));
         if (L.accumIdStart + s0 + a == 0) {
@@ -2500,6 +2510,7 @@ inline gbv_status launch_render_noalloc(RenderParams p, const Store &store, cuda
   // blocks per SM, the default traversal settings, no shared-memory staging
   p.skip = kSkipDefault;
   p.threshold = kThresholdDefault;
+  p.idlePolls = kIdlePolls;
   p.maskWords = 0;
   p.cdfYOff = p.pivOff = p.rowOff = -1;
   p.pivPerRow = 0;

@@ -177,3 +177,26 @@ def test_background_taken_in_groups_equals_wavefront(cuda, kind):
     torch.cuda.synchronize()
     for a in [acc, whole(g, 3)] + list(batch.accums):
         np.testing.assert_array_equal(bits(a.cpu().numpy()), bits(ref.cpu().numpy()))
+
+
+@pytest.mark.parametrize("kind", ["single", "multi", "iso"])
+@pytest.mark.parametrize("counted", [True, False])
+def test_warps_that_give_up_are_reported(cuda, kind, counted):
+    """The frame kernel's limit on a warp's looks for work, set so low that
+    warps reach it while other warps' paths are under way: the frame may lack
+    pixels, and the launch says so; with the limit out of reach it does not."""
+    import torch
+    g = GpuScene(world(kind, 640, 360))
+    ref = g.render(spp=4)
+    for polls in (0, 1 << 20):
+        acc = g.new_accum()
+        counters = torch.zeros(N.GBV_NUM_COUNTERS, dtype=torch.int64, device="cuda") if counted else None
+        flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+        N.check(N.lib().gbv_selftest_idle_limit(C.byref(g.record()), _ptr(acc), 640, 360, 4, polls, _ptr(counters),
+                                                _ptr(flag), _stream()), "gbv_selftest_idle_limit")
+        torch.cuda.synchronize()
+        assert flag.item() == (polls == 0)
+        if counted:
+            assert (counters[N.GBV_COUNTER_CAPS].item() > 0) == (polls == 0)
+        if polls:
+            np.testing.assert_array_equal(bits(acc.cpu().numpy()), bits(ref.cpu().numpy()))
