@@ -1484,7 +1484,10 @@ template <bool Iso> struct PathPool {
     const int mine = min(max(want - before, 0), c);
     const uint32_t sel = mine == c ? bits : bits & ((1u << nth_bit(bits, mine)) - 1u);
     const uint32_t got = sel ? atomicAnd(const_cast<uint32_t *>(m) + at, ~sel) & sel : 0u;
+    // the lane that took a path is seldom the one that reads its record: the
+    // barrier orders their accesses (the shuffles below order no memory)
     __threadfence_block();
+    __syncwarp();
     const int g = __popc(got), upTo = warp_scan(g);
     n = __shfl_sync(FULL, upTo, 31);
     const int first = upTo - g;
