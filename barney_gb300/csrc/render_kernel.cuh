@@ -2343,6 +2343,14 @@ inline size_t staged_words(const RenderParams &p) {
 
 using RenderKernelFn = void (*)(const RenderParams, const RenderParams *, const long long *, int, int *);
 
+// The words plan_staging places at most (64 KB of tables, the row terms on top
+// where the bitmask fills them), and the shared memory a launch may ask for:
+// the kernel's limit is always set to this, whatever one launch needs, since
+// another host thread may set it for its own scene before this one's launch.
+constexpr int kMaxStagedWords = 16 * 1024 + 2 * 1024 + 4;
+template <bool Iso> constexpr size_t kMaxDynamicSmem = (kMaxStagedWords + PathPool<Iso>::kStride) * sizeof(uint32_t);
+static_assert(kMaxDynamicSmem<true> + 1024 <= 227 * 1024, "a block's tables and path pool");
+
 // Places the block's path pool behind the `staged` words of tables; returns
 // the block's dynamic shared memory in bytes.
 template <bool Iso> inline size_t plan_pool(RenderParams &p, size_t staged) {
@@ -2353,12 +2361,13 @@ template <bool Iso> inline size_t plan_pool(RenderParams &p, size_t staged) {
 // Persistent grid of a launch over `tiles` warp tiles: one block per SM, and
 // the path slots each block uses: no more than its share of the pixels, so
 // that no block holds pixels that another would be idle without.
-inline gbv_status plan_grid(RenderParams &p, RenderKernelFn kernel, size_t smem, long long tiles, long long &blocks) {
+inline gbv_status plan_grid(RenderParams &p, RenderKernelFn kernel, size_t smemLimit, long long tiles,
+                            long long &blocks) {
   int dev = 0, sms = 0;
   gbv_status st = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
   if (st == GBV_OK) st = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-  if (st == GBV_OK && smem > 48 * 1024)
-    st = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+  if (st == GBV_OK)
+    st = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemLimit),
                     "render_kernel: shared-memory size");
   if (st != GBV_OK) return st;
   blocks = tiles < sms ? tiles : sms;
@@ -2390,6 +2399,7 @@ inline gbv_status launch_render_t(const RenderParams &p, const Store &store, cud
   const RenderKernelFn kernel = p.counters ? kCount : kPlain;
   RenderParams q = p;
   const size_t smem = p.isoOn ? plan_pool<true>(q, staged_words(p)) : plan_pool<false>(q, staged_words(p));
+  const size_t limit = p.isoOn ? kMaxDynamicSmem<true> : kMaxDynamicSmem<false>;
   long long blocks = 0;
   gbv_status st = GBV_OK;
   // the tile pool counter, the majorant bitmask and the log live in
@@ -2420,7 +2430,7 @@ inline gbv_status launch_render_t(const RenderParams &p, const Store &store, cud
     q.spp = p.spp - done < step ? p.spp - done : step;
     if (plan_split(q, inner, outer, logBytes ? hits : 1, logBytes ? kLogBytes : 0))
       q.log = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(pool) + 256 + maskBytes);
-    st = plan_grid(q, kernel, smem, launch_tiles(q), blocks);
+    st = plan_grid(q, kernel, limit, launch_tiles(q), blocks);
     if (st == GBV_OK)
       st = check_cuda(cudaMemsetAsync(pool, 0, 2 * sizeof(int), stream), "render_kernel: clearing the tile pool");
     if (st == GBV_OK) {
@@ -2526,7 +2536,8 @@ inline gbv_status launch_render_noalloc(RenderParams p, const Store &store, cuda
   const RenderKernelFn kernel = p.counters ? kCount : kPlain;
   const size_t smem = p.isoOn ? plan_pool<true>(p, 0) : plan_pool<false>(p, 0);
   long long blocks = 0;
-  gbv_status st = plan_grid(p, kernel, smem, launch_tiles(p), blocks);
+  gbv_status st = plan_grid(p, kernel, p.isoOn ? kMaxDynamicSmem<true> : kMaxDynamicSmem<false>, launch_tiles(p),
+                            blocks);
   if (st != GBV_OK) return st;
   st = check_cuda(cudaMemsetAsync(pool, 0, 2 * sizeof(int), stream), "gbv_render_noalloc: clearing the tile pool");
   if (st != GBV_OK) return st;
@@ -2563,7 +2574,7 @@ inline gbv_status batch_launch_t(const gbv_batch *b, RenderParams L, cudaStream_
   // by themselves: 64 scenes 0.82 -> 0.80 ms without the log
   const size_t room = L.spp > 1 ? b->logBytes : 0;
   if (plan_split(L, b->innerTiles, b->outerTiles, b->hits, room)) L.log = b->d_log;
-  gbv_status st = plan_grid(L, kernel, smem, launch_tiles(L), blocks);
+  gbv_status st = plan_grid(L, kernel, kMaxDynamicSmem<false>, launch_tiles(L), blocks);
   if (st == GBV_OK) st = check_cuda(cudaMemsetAsync(b->d_pool, 0, 2 * sizeof(int), stream), "gbv_batch_render: pool");
   if (st != GBV_OK) return st;
   kernel<<<(unsigned)blocks, block_threads(Budget), smem, stream>>>(L, b->d_items, b->d_tileStart, b->count, b->d_pool);

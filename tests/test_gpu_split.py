@@ -6,7 +6,9 @@ gbv_render_noalloc has no log and splits none.  The sizes are the edges: one
 pixel, part of a warp tile, one tile, one tile and a column and a row, and
 frames whose log has room for part of the tiles or for none."""
 import ctypes as C
+import subprocess
 import threading
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -137,6 +139,41 @@ def test_scratch_is_safe_across_threads_and_streams(cuda):
     for ref, frames in zip(refs, out):
         for f in frames:
             np.testing.assert_array_equal(bits(f), bits(ref))
+
+
+def test_threads_render_scenes_of_other_tables(cuda, tmp_path):
+    """Threads render scenes whose shared-memory tables differ in size (few
+    and many macrocells, without an env map and with low and high ones,
+    without tables at all): no call fails, and every frame is the one a lone
+    launch renders."""
+    import torch
+    root = Path(__file__).resolve().parent.parent
+    lib = tmp_path / "librender_threads.so"
+    r = subprocess.run(["gcc", "-std=c99", "-O2", "-fPIC", "-shared", "-I", str(root / "include"),
+                        str(root / "tests" / "c" / "render_threads.c"), "-L", str(root / "barney_gb300" / "_lib"),
+                        "-lbarney_gb300", f"-Wl,-rpath,{root / 'barney_gb300' / '_lib'}", "-lpthread", "-o", str(lib)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    gs = []
+    for dims, cells, env in ((16, 8, 0), (64, 2, 0), (16, 8, 1000), (64, 2, 32), (48, 4, 300), (64, 2, 0)):
+        s = scenes.small_scene(dims=dims, spp=1, width=16, height=8)
+        s.cells_per_mc = cells
+        if env:
+            s.env = scenes.env_sky(64, env)
+        gs.append(GpuScene(s))
+    n = len(gs)
+    refs = [whole(g, 1).cpu().numpy() for g in gs]
+    accums, streams = [g.new_accum() for g in gs], [torch.cuda.Stream() for _ in gs]
+    torch.cuda.synchronize()
+    records = [g.record() for g in gs]
+    message = C.create_string_buffer(256)
+    failed = C.CDLL(str(lib)).render_threads(
+        (N.GbvScene * n)(*records), (C.c_void_p * n)(*[a.data_ptr() for a in accums]),
+        (C.c_void_p * n)(*[st.cuda_stream for st in streams]), N.ivec(*[0] * (n - 1), 1), n, 16, 8, 2000, message)
+    torch.cuda.synchronize()
+    assert failed == 0, (failed, message.value.decode())
+    for a, ref in zip(accums, refs):
+        np.testing.assert_array_equal(bits(a.cpu().numpy()), bits(ref))
 
 
 def test_captured_render_replays(cuda):
