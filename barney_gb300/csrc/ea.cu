@@ -408,7 +408,9 @@ __device__ __forceinline__ void flush8(float *__restrict__ dst, bool flush, unsi
 // memory until it is done.  A block per 16x8 pixels waited at its end for its
 // longest ray (1.25 of 8.6 stall cycles) and cleared and flushed the gradient
 // for every patch: 32 views of 256^2 through 128^3, 2168 us; this takes 1910.
-template <int MinBlocks>
+// Without a counter (Counted = false) a warp takes one tile, and the grid has a
+// block per four tiles.
+template <int MinBlocks, bool Counted>
 __global__ void __launch_bounds__(128, MinBlocks) ea_backward_kernel(const EAParams p, const float4 *__restrict__ img,
                                                           const float4 *__restrict__ gimg, float *__restrict__ gvox,
                                                           float *__restrict__ gtf, int *__restrict__ counter) {
@@ -417,10 +419,12 @@ __global__ void __launch_bounds__(128, MinBlocks) ea_backward_kernel(const EAPar
   for (int i = threadIdx.x; i < ntf; i += blockDim.x) s_gtf[i] = 0.f;
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  while (true) {
-    int tile = 0;
-    if (lane == 0) tile = atomicAdd(counter, 1);
-    tile = __shfl_sync(0xffffffffu, tile, 0);
+  do {
+    int tile = 4 * blockIdx.x + (threadIdx.x >> 5);
+    if (Counted) {
+      if (lane == 0) tile = atomicAdd(counter, 1);
+      tile = __shfl_sync(0xffffffffu, tile, 0);
+    }
     if (tile >= p.tileStart[p.numViews]) break;
     int view = 0;
     while (tile >= p.tileStart[view + 1]) view++;
@@ -572,7 +576,7 @@ __global__ void __launch_bounds__(128, MinBlocks) ea_backward_kernel(const EAPar
         tAcc[7] += dsb * f;
       }
     }
-  }
+  } while (Counted);
   __syncthreads();
   for (int i = threadIdx.x; i < ntf; i += blockDim.x)
     if (s_gtf[i] != 0.f) atomicAdd(gtf + i, s_gtf[i]);
@@ -636,7 +640,7 @@ static gbv_status ea_prepare(const gbv_scene *s, float step, EAParams &p, bool f
 //   field);
 // * a field of few blocks has few empty ones (32^3, 16 views of 320^2: 165 us
 //   against 159; 64^3, 8 views of 512^2: 321 against 365).
-// Without scratch the march takes every step.
+// Without scratch, and in a capture, the march takes every step.
 constexpr double kSkipPixels = 768. * 1024.;
 constexpr int kSkipCells = 48;
 static gbv_status find_empty(const gbv_scene *s, EAParams &p, const gbv_ea_view *views, int num_views, void **scratch,
@@ -659,11 +663,7 @@ static gbv_status find_empty(const gbv_scene *s, EAParams &p, const gbv_ea_view 
   for (int i = 0; i < 3; i++) p.eb[i] = M[i];
   const size_t blocks = (size_t)M[0] * M[1] * M[2];
   const size_t head = (sizeof(EmptyBlocks) + blocks + 255) & ~(size_t)255;
-  if (scratch_alloc(scratch, head + (linear ? blocks * sizeof(float2) : 0), cs) != cudaSuccess) {
-    cudaGetLastError();
-    *scratch = nullptr;
-    return GBV_OK;
-  }
+  if (!optional_scratch(scratch, head + (linear ? blocks * sizeof(float2) : 0), cs)) return GBV_OK;
   EmptyBlocks *out = static_cast<EmptyBlocks *>(*scratch);
   gbv_status st = check_cuda(cudaMemsetAsync(out, 0, 16, cs), "gbv_ea_render: scratch");
   if (st == GBV_OK && linear) {
@@ -682,7 +682,7 @@ static gbv_status find_empty(const gbv_scene *s, EAParams &p, const gbv_ea_view 
     st = check_launch("empty_kernel");
   }
   if (st == GBV_OK) p.empty = out;
-  else cudaFreeAsync(*scratch, cs), *scratch = nullptr;
+  else free_optional_scratch(*scratch, cs), *scratch = nullptr;
   return st;
 }
 
@@ -746,11 +746,8 @@ gbv_status gbv_ea_render(const gbv_scene *s, const gbv_ea_view *views, int num_v
 #undef GBV_EA_FORWARD
     return check_launch("ea_forward_kernel");
   });
-  if (scratch) {
-    const gbv_status fst = check_cuda(cudaFreeAsync(scratch, (cudaStream_t)stream), "gbv_ea_render: scratch");
-    if (st == GBV_OK) st = fst;
-  }
-  return st;
+  const gbv_status fst = check_cuda(free_optional_scratch(scratch, (cudaStream_t)stream), "gbv_ea_render: scratch");
+  return st != GBV_OK ? st : fst;
 }
 
 gbv_status gbv_ea_render_f64(const gbv_scene *s, const gbv_ea_view *views, int num_views, float step,
@@ -784,26 +781,29 @@ gbv_status gbv_ea_backward_ex(const gbv_scene *s, const gbv_ea_view *views, int 
   int dev = 0, sms = 0;
   st = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
   if (st == GBV_OK) st = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-  // a tile counter per launch
+  if (st != GBV_OK) return st;
+  // a tile counter per launch, if there is scratch
   const int launches = (num_views + kMaxViewsPerLaunch - 1) / kMaxViewsPerLaunch;
   int *counters = nullptr;
   cudaStream_t cs = (cudaStream_t)stream;
-  if (st == GBV_OK) st = check_cuda(scratch_alloc((void **)&counters, sizeof(int) * launches, cs), "gbv_ea_backward: scratch");
-  if (st != GBV_OK) return st;
-  st = check_cuda(cudaMemsetAsync(counters, 0, sizeof(int) * launches, cs), "gbv_ea_backward: scratch");
+  if (optional_scratch((void **)&counters, sizeof(int) * launches, cs))
+    st = check_cuda(cudaMemsetAsync(counters, 0, sizeof(int) * launches, cs), "gbv_ea_backward: scratch");
   int launch = 0;
   if (st == GBV_OK)
     st = for_view_chunks(p, views, num_views, [&](EAParams &q, int cnt, int, int) {
-      const int tiles = q.tileStart[cnt], grid = std::min(sms * occ, (tiles + 3) / 4);
+      const int tiles = q.tileStart[cnt], blocks = (tiles + 3) / 4, grid = counters ? std::min(sms * occ, blocks) : blocks;
       const float4 *img = reinterpret_cast<const float4 *>(d_images);
       const float4 *gimg = reinterpret_cast<const float4 *>(d_grad_images);
-      int *counter = counters + launch++;
-      if (occ == 8) ea_backward_kernel<8><<<grid, 128, smem, cs>>>(q, img, gimg, d_grad_scalars, d_grad_tf, counter);
-      else if (occ == 6) ea_backward_kernel<6><<<grid, 128, smem, cs>>>(q, img, gimg, d_grad_scalars, d_grad_tf, counter);
-      else ea_backward_kernel<4><<<grid, 128, smem, cs>>>(q, img, gimg, d_grad_scalars, d_grad_tf, counter);
+      int *counter = counters ? counters + launch++ : nullptr;
+      const auto launch_as = [&](auto kernel) {
+        kernel<<<grid, 128, smem, cs>>>(q, img, gimg, d_grad_scalars, d_grad_tf, counter);
+      };
+      if (occ == 8) counter ? launch_as(ea_backward_kernel<8, true>) : launch_as(ea_backward_kernel<8, false>);
+      else if (occ == 6) counter ? launch_as(ea_backward_kernel<6, true>) : launch_as(ea_backward_kernel<6, false>);
+      else counter ? launch_as(ea_backward_kernel<4, true>) : launch_as(ea_backward_kernel<4, false>);
       return check_launch("ea_backward_kernel");
     });
-  const gbv_status fst = check_cuda(cudaFreeAsync(counters, cs), "gbv_ea_backward: scratch");
+  const gbv_status fst = check_cuda(free_optional_scratch(counters, cs), "gbv_ea_backward: scratch");
   return st != GBV_OK ? st : fst;
 }
 

@@ -18,6 +18,12 @@ gbv_status launch_mc_ranges(const float *d_scalars, const int dims[3], int cpm, 
 // Stream-ordered scratch of a launch from the library's pool of the current
 // device (scratch.cpp); returned with cudaFreeAsync.
 cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
+// Scratch that a launch can do without: false (and *ptr null) where there is
+// none, and while the stream is captured -- a graph that allocates can be
+// neither cloned nor put into another one, and has one instance at a time.
+// May be called while another stream is captured.
+bool optional_scratch(void **ptr, size_t bytes, cudaStream_t stream);
+cudaError_t free_optional_scratch(void *ptr, cudaStream_t stream);
 
 // The device view of a parsed NanoVDB grid whose buffer is at d_grid
 // (nanovdb.cu).

@@ -64,4 +64,32 @@ cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream) {
   return cudaMallocAsync(ptr, bytes, stream);
 }
 
+namespace {
+// This thread's calls may allocate although another stream is being captured
+// (which they do not touch), whatever that capture's mode.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+}  // namespace
+
+bool optional_scratch(void **ptr, size_t bytes, cudaStream_t stream) {
+  const RelaxedCapture relaxed;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  *ptr = nullptr;
+  cudaError_t e = cudaStreamIsCapturing(stream, &cap);
+  if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) return false;
+  if (e == cudaSuccess) e = scratch_alloc(ptr, bytes, stream);
+  if (e == cudaSuccess) return true;
+  cudaGetLastError();
+  *ptr = nullptr;
+  return false;
+}
+
+cudaError_t free_optional_scratch(void *ptr, cudaStream_t stream) {
+  const RelaxedCapture relaxed;
+  return ptr ? cudaFreeAsync(ptr, stream) : cudaSuccess;
+}
+
 }  // namespace gbv

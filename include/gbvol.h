@@ -460,7 +460,11 @@ typedef struct gbv_ea_view {
    width*height RGBA float).  FP32 interpolation and transmittance with
    compensated optical depth.  The field is FP32 LINEAR or a brick-corner
    store of any format and brick shape (FP16/BF16/U8 voxels are widened to
-   FP32 before interpolation). */
+   FP32 before interpolation).
+   Large launches take scratch (1 to 9 bytes per 64 or 512 cells) to skip
+   empty space, and gbv_ea_backward 4 bytes per 32 views, both in `stream`
+   order.  Where there is none, and in a stream capture, they do without it:
+   the same image, and the gradients of another order of additions, slower. */
 gbv_status gbv_ea_render(const gbv_scene *scene, const gbv_ea_view *views,
                          int num_views, float step, float *d_images,
                          void *stream);

@@ -394,6 +394,98 @@ def test_adjoint_of_an_infinite_transmittance(cuda):
     assert np.isnan(gt.cpu().numpy()[3:]).all()
 
 
+def _search_case():
+    """A march of enough pixels to look for empty blocks, and gradients of its images."""
+    import torch
+    s = scenes.Scene(scalars=scenes.blob_volume((64, 64, 64), 12, seed=8, noise=0.0), tf=scenes.tf_two_peaks(256),
+                     base_density=20.0)
+    views = scenes.fibonacci_views(4, 2.5, 8)
+    for v in views:
+        v["width"], v["height"] = 640, 400
+    p = EAProblem(s, views, 0.5 / 63)
+    img = p.render()
+    gimg = torch.rand(img.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    torch.cuda.synchronize()
+    return p, img, gimg
+
+
+class _Calls:
+    """gbv_ea_render and gbv_ea_backward into buffers of their own, and what they are to hold."""
+
+    def __init__(self, p, img, gimg):
+        import torch
+        self.p, self.img, self.gimg = p, img, gimg
+        self.gv, self.gt = p.backward(img, gimg)
+        self.out, self.cv, self.ct = torch.empty_like(img), torch.zeros_like(self.gv), torch.zeros_like(self.gt)
+        self.rec = p.record()
+
+    def clear(self):
+        import torch
+        for t in (self.out, self.cv, self.ct):
+            t.zero_()
+        torch.cuda.synchronize()
+
+    def run(self, stream):
+        import ctypes as C
+        p, n = self.p, len(self.p.views)
+        N.check(N.lib().gbv_ea_render(C.byref(self.rec), p._views_c, n, p.step, self.out.data_ptr(), stream))
+        N.check(N.lib().gbv_ea_backward(C.byref(self.rec), p._views_c, n, p.step, self.img.data_ptr(),
+                                        self.gimg.data_ptr(), self.cv.data_ptr(), self.ct.data_ptr(), stream))
+
+    def check(self):
+        import torch
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(self.out.cpu().numpy().view(np.uint32), self.img.cpu().numpy().view(np.uint32))
+        # the gradients' additions may be in another order: each entry's
+        # rounding is far below 1e-5 of the largest
+        for got, ref in ((self.cv, self.gv), (self.ct, self.gt)):
+            np.testing.assert_allclose(got.cpu(), ref.cpu(), rtol=1e-4, atol=1e-5 * float(ref.abs().max()))
+
+
+def _runtime():
+    import ctypes as C
+    return C.CDLL(next(x.split()[-1] for x in open("/proc/self/maps") if "libcudart" in x))
+
+
+def test_captured_march_and_adjoint(cuda):
+    """A capture of the march and its adjoint holds kernels alone: the graph
+    can be cloned, put into another one and instantiated twice, and each
+    replay gives the calls' results."""
+    import ctypes as C
+    import torch
+    rt, calls = _runtime(), _Calls(*_search_case())
+    stream = torch.cuda.Stream()
+    st = C.c_void_p(stream.cuda_stream)
+    graph, clone, parent, node = C.c_void_p(), C.c_void_p(), C.c_void_p(), C.c_void_p()
+    assert rt.cudaStreamBeginCapture(st, 1) == 0
+    calls.run(st)
+    assert rt.cudaStreamEndCapture(st, C.byref(graph)) == 0
+    assert rt.cudaGraphClone(C.byref(clone), graph) == 0
+    assert rt.cudaGraphCreate(C.byref(parent), 0) == 0
+    assert rt.cudaGraphAddChildGraphNode(C.byref(node), parent, None, C.c_size_t(0), graph) == 0
+    for g in (graph, graph, clone, parent):
+        exe = C.c_void_p()
+        assert rt.cudaGraphInstantiate(C.byref(exe), g, C.c_ulonglong(0)) == 0
+        calls.clear()
+        assert rt.cudaGraphLaunch(exe, st) == 0
+        calls.check()
+
+
+def test_march_and_adjoint_beside_a_capture(cuda):
+    """The calls on one stream while another one is captured, in the mode that
+    forbids allocations: both go on."""
+    import ctypes as C
+    import torch
+    rt, calls = _runtime(), _Calls(*_search_case())
+    other, mine = torch.cuda.Stream(), torch.cuda.Stream()
+    graph = C.c_void_p()
+    calls.clear()
+    assert rt.cudaStreamBeginCapture(C.c_void_p(other.cuda_stream), 0) == 0
+    calls.run(C.c_void_p(mine.cuda_stream))
+    assert rt.cudaStreamEndCapture(C.c_void_p(other.cuda_stream), C.byref(graph)) == 0
+    calls.check()
+
+
 @pytest.mark.parametrize("w,h,nviews", [(1, 1, 1), (9, 5, 3), (33, 17, 2), (16, 8, 33)])
 def test_adjoint_tiles_of_uneven_views(cuda, w, h, nviews):
     """Views whose tiles are partial, and more of them than one launch holds:
