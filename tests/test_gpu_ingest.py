@@ -51,6 +51,15 @@ def test_macrocell_ranges_at_strip_edges(cuda, dims, cpm):
     np.testing.assert_array_equal(bits(out.cpu().numpy()), bits(want))
 
 
+@pytest.mark.parametrize("nx", [2, 3, 5, 9, 16, 17, 33, 63, 64])
+@pytest.mark.parametrize("cpm", [1, 2, 3, 4, 8, 16, 31, 64, 200])
+def test_macrocell_ranges_of_thin_fields(cuda, nx, cpm):
+    """Fields of few voxels along x: blocks that hold several rows of
+    macrocells, the last one fewer; slices of one row and of many."""
+    test_macrocell_ranges_at_strip_edges(cuda, (nx, 43, 37), cpm)
+    test_macrocell_ranges_at_strip_edges(cuda, (nx, 2, 67), cpm)
+
+
 @pytest.mark.parametrize("bits_,shift", [(8, 0), (8, 3), (16, 0), (16, 2)])
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 4096, 4099])
 def test_normalized_texels_at_vector_edges(cuda, bits_, shift, n):
