@@ -91,6 +91,7 @@ def lib() -> C.CDLL:
         sig = {
             "gbv_last_error": (C.c_char_p, []),
             "gbv_version": (i, []),
+            "gbv_release_scratch": (st, []),
             "gbv_mc_dims": (st, [ip, i, ip]),
             "gbv_build_mc_ranges": (st, [vp, ip, i, vp, vp]),
             "gbv_build_mc_ranges_from_store": (st, [vp, vp, i, ip, i, vp, vp]),

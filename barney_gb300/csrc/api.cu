@@ -294,6 +294,12 @@ extern "C" {
 const char *gbv_last_error(void) { return g_last_error.c_str(); }
 int gbv_version(void) { return 1; }
 
+gbv_status gbv_release_scratch(void) {
+  int dev = 0;
+  const gbv_status st = check_cuda(cudaGetDevice(&dev), "gbv_release_scratch");
+  return st != GBV_OK ? st : check_cuda(release_scratch(dev), "gbv_release_scratch");
+}
+
 gbv_status gbv_mc_dims(const int dims[3], int cells_per_mc, int mc_dims[3]) {
   if (!dims || !mc_dims || cells_per_mc <= 0) return set_error(GBV_ERROR_INVALID_ARGUMENT, "gbv_mc_dims: bad argument");
   for (int i = 0; i < 3; i++) {

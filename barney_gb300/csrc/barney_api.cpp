@@ -656,9 +656,11 @@ BNContext bnContextCreate(const int *dataRanks, int numDataRanks, const int *gpu
 
 void bnContextDestroy(BNContext context) {
   Context *c = (Context *)context;
+  bool last = true;  // the device's last context
   {
     std::lock_guard<std::mutex> lock(g_mutex);
     if (!g_contexts.erase(c)) return;
+    for (const Context *other : g_contexts) last = last && other->device != c->device;
   }
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
@@ -666,6 +668,7 @@ void bnContextDestroy(BNContext context) {
   cudaStreamSynchronize(c->stream);
   if (c->mem.pool) cudaMemPoolDestroy(c->mem.pool);
   cudaStreamDestroy(c->stream);
+  if (last) gbv::release_scratch(c->device);
   delete c;
 }
 

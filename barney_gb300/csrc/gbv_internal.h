@@ -18,6 +18,8 @@ gbv_status launch_mc_ranges(const float *d_scalars, const int dims[3], int cpm, 
 // Stream-ordered scratch of a launch from the library's pool of the current
 // device (scratch.cpp); returned with cudaFreeAsync.
 cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream);
+// Gives the pool's memory that no launch holds back to the device.
+cudaError_t release_scratch(int dev);
 // Scratch that a launch can do without: false (and *ptr null) where there is
 // none, and while the stream is captured -- a graph that allocates can be
 // neither cloned nor put into another one, and has one instance at a time.

@@ -350,9 +350,9 @@ extern "C" gbv_status gbv_tile_partition(int width, int height, int rank, int nu
 // render: an application that hands out all HBM from its own pre-sized pool
 // and requires libraries to work inside the buffers it passes them, or a
 // real-time viewer that forbids allocation and free calls on its frame
-// path (gbv_render takes its scratch from cudaMallocAsync and
-// returns it with cudaFreeAsync, which draw on the device's memory pool).
-// This entry point takes its scratch, two words, from a file-scope device array
+// path (gbv_render takes its scratch, a long frame's up to 512 MB, from the
+// library's memory pool and keeps it there).  This entry point takes its
+// scratch, two words, from a file-scope device array
 // instead.
 // ===========================================================================
 namespace gbv {

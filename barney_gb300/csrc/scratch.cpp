@@ -6,7 +6,8 @@
 // scratch anew: 40-100 us of host time per gbv_render (GB300, 256 bytes of
 // scratch).  The pool orders reuse by the streams' own work, is safe to use
 // from several threads and streams, and does not make one stream wait for
-// another to reuse its memory.
+// another to reuse its memory.  The largest request is a frame's fragment log
+// (512 MB); release_scratch gives back what no launch holds.
 #include <mutex>
 #include <cuda_runtime.h>
 #include "gbv_internal.h"
@@ -20,8 +21,8 @@ std::mutex g_mutex;
 cudaMemPool_t g_pools[kMaxDevices];
 
 // The pool of device `dev` (made on first use); null if it cannot be made.
-// `stale`: a pool that failed, to be made anew (a device reset destroys
-// pools behind their handles).
+// `stale`: a pool whose handle is no longer valid (a device reset destroys
+// pools behind their handles), to be made anew.
 cudaMemPool_t device_pool(int dev, cudaMemPool_t stale) {
   if (dev < 0 || dev >= kMaxDevices) return nullptr;
   std::lock_guard<std::mutex> lock(g_mutex);
@@ -57,11 +58,20 @@ cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream) {
   cudaMemPool_t pool = cap == cudaStreamCaptureStatusNone ? device_pool(dev, nullptr) : nullptr;
   for (int attempt = 0; pool && attempt < 2; attempt++) {
     e = cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
-    if (e == cudaSuccess || e == cudaErrorMemoryAllocation) return e;
+    if (e != cudaErrorInvalidValue && e != cudaErrorInvalidResourceHandle) return e;  // the handle is valid
     cudaGetLastError();
     pool = device_pool(dev, pool);
   }
   return cudaMallocAsync(ptr, bytes, stream);
+}
+
+cudaError_t release_scratch(int dev) {
+  cudaMemPool_t pool = nullptr;
+  if (dev >= 0 && dev < kMaxDevices) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    pool = g_pools[dev];
+  }
+  return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
 }
 
 namespace {

@@ -50,6 +50,14 @@ enum { GBV_ADDR_WRAP = 0, GBV_ADDR_CLAMP = 1, GBV_ADDR_BORDER = 2, GBV_ADDR_MIRR
 const char *gbv_last_error(void);
 int gbv_version(void);
 
+/* Gives the scratch memory that the library keeps on the current device, and
+   that no launch holds, back to the device.  Launches take their scratch in
+   stream order from a pool of the library's own, which keeps up to 576 MB per
+   device between them: a frame's fragment log takes up to 512 MB (see
+   gbv_render), everything else a few MB.  bnContextDestroy does the same with
+   the device's last context. */
+gbv_status gbv_release_scratch(void);
+
 /* ------------------------------------------------------------------------
  * Macrocells.
  * ------------------------------------------------------------------------ */
@@ -302,6 +310,11 @@ gbv_status gbv_env_build_cdfs(const float *d_texels, int width, int height,
    row 0 the bottom row), accumulating as the reference does: the first pass
    of a fresh frame (accum_id_start == 0) overwrites.  d_counters: optional,
    GBV_NUM_COUNTERS uint64 (accumulated, not cleared).
+   Scratch: up to 8 KB, and for frames without depth and ID channels a log of
+   the passes' fragments, 20 to 140 bytes per pixel and pass of the tiles that
+   may see the field, at most 512 MB per call in flight (a captured call's
+   belongs to its graph); without room for the log the same frame is rendered
+   without it.
    Replaces Context::renderTiles' generate/trace/shade loop
    (barney/Context.cpp:142-185; barney/kernels/generateRays.cu:44-243,
    traceRays.dev.cu:20-52, shadeRays.cu:881-1041;
