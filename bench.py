@@ -565,9 +565,10 @@ def batch_timing(count=64, reps=3):
     return out
 
 
-def own_launches(call) -> int:
-    """Kernel launches of this library in one call (counted in an untimed call;
-    a profiler's first session may record nothing, hence two)."""
+def own_launches(call):
+    """Kernel launches of this library in one call, counted by the profiler in
+    an untimed call (its first session may record nothing, hence two); None
+    where it recorded none."""
     import torch
     from torch.profiler import ProfilerActivity, profile
     n = 0
@@ -576,9 +577,7 @@ def own_launches(call) -> int:
             call()
             torch.cuda.synchronize()
         n = sum(1 for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA and "gbv::" in e.name)
-    # where the profiler cannot run: the mask kernel, three parts
-    # (profiles/launches_bench_512cube_1080p_64spp.md)
-    return n or 7
+    return n or None
 
 
 def run_ours(args):
@@ -642,6 +641,7 @@ def run_ours(args):
         # scale the captured launch's DRAM bytes by density samples processed
         if t.get("format") == args.format and t.get("samples"):
             traffic = t["dram_bytes"] * samples / t["samples"]
+    launches = own_launches(frame)
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": frame_ms, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
@@ -655,8 +655,9 @@ def run_ours(args):
                          else "fallback 6800 GB/s",
                          "bytes_per_launch": bytes_launch, "kernel": "render_kernel"},
             # per frame: the majorant-bitmask kernel, then per part of the
-            # frame's passes the render kernel and the log's resolve kernel
-            "gpu_launches": own_launches(frame) * args.steps, "clocks": clk.summary()}
+            # frame's passes the render kernel and the kernel that finishes
+            # the part (null: not observed)
+            "gpu_launches": launches and launches * args.steps, "clocks": clk.summary()}
     # ---- e2e through the bn* C-ABI with host buffers, on every rank; the
     # slowest rank's step time counts ----
     if world > 1:
