@@ -207,7 +207,7 @@ static bool resolve_config(const gbv_render_config *c, RenderParams &p, LaunchCh
   lc.stage = c->stage;
   if (c->threshold_pct) p.threshold = c->threshold_pct;
   else if (c->mode == GBV_RENDER_WAVEFRONT) p.threshold = 25;
-  if (c->skip_cells) p.skip = c->skip_cells;
+  if (c->skip_cells) p.skip = lc.skip = c->skip_cells;
   p.profile = c->profile;
   return true;
 }

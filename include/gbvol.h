@@ -328,13 +328,14 @@ gbv_status gbv_render(const gbv_scene *scene, float *d_accum, int width,
    default, so a zero-initialised struct (or a null pointer) is the default
    launch.
    blocks_per_sm: the register budget, as resident 128-thread blocks per SM:
-     4 (128 registers a thread), 5 or 6; by default 4, or 5 for long frames.
+     4 (128 registers a thread), 5 or 6; by default 4, 5 for long frames and 6
+     for long single-scatter ones that the field fills.
      The persistent kernel runs one block of that many threads on each SM.
    threshold_pct: a warp keeps tracing while at least this percentage of its
      lanes is (1..100, default 25), or while no other stage has work for it.
    skip_cells: rounds (a cell test, a Woodcock distance draw and a step) a
      lane makes per traversal iteration before the warp samples (1..1024,
-     default 4).
+     default 4, or 8 with a budget of 6 by default).
    stage: shared-memory staging, GBV_STAGE_DEFAULT (the bitmask of non-zero
      majorants, at most 8 KB, computed once per launch in HBM and copied to
      each block by one bulk copy, and the env map's per-row pdf terms),
