@@ -447,6 +447,26 @@ def _runtime():
     return C.CDLL(next(x.split()[-1] for x in open("/proc/self/maps") if "libcudart" in x))
 
 
+@pytest.mark.parametrize("fmt", [None, N.GBV_VOXEL_F16])
+def test_empty_blocks_are_looked_for(cuda, fmt):
+    """The four views of the tests that compare the two marches call for the
+    search, one of them alone does not."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    from barney_gb300.device import GpuScene
+    p, _, _ = _search_case()
+    store = GpuScene(p.s, fmt=fmt) if fmt is not None else None
+    for views, searches in ((p.views, 1), (p.views[:1], 0)):
+        q = EAProblem(p.s, views, p.step, store=store)
+        for _ in range(2):  # a profiler's first session may record nothing
+            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+                q.render()
+                torch.cuda.synchronize()
+            names = [e.name for e in prof.events() if "gbv::" in e.name]
+        assert sum("ea_forward_kernel" in n for n in names) == 1
+        assert sum("empty_kernel" in n or "empty_ranges_kernel" in n for n in names) == searches
+
+
 def test_captured_march_and_adjoint(cuda):
     """A capture of the march and its adjoint holds kernels alone: the graph
     can be cloned, put into another one and instantiated twice, and each
