@@ -246,12 +246,19 @@ __global__ void tonemap_kernel(const float4 *__restrict__ accum, long long n, fl
 // CUDA texture objects, rtcore/cudaCommon/TextureData.cu:34-39; the CPU
 // backend's getTexel<unsigned char>, rtcore/embree/Texture.cpp:216-225):
 // v / 255 or v / 65535, one IEEE division per texel.
-// A thread takes 16 bytes of texels where both arrays are 16-byte aligned,
-// and the remainder one by one.  What bounds it: memory.  One texel a thread
-// took 46 us for 16.8 M 8-bit texels (1.8 TB/s); this takes 21 us (4.0).
+// What bounds it: memory.  One texel a thread took 46 us for 16.8 M 8-bit texels
+// (1.8 TB/s); 16 bytes of them a thread takes 21 us (4.0).
 template <typename T>
-__global__ void __launch_bounds__(256) normalize_texels_kernel(const T *__restrict__ in, long long n, long long vectors,
-                                                               float scale_max, float *__restrict__ out) {
+__global__ void __launch_bounds__(256) normalize_texels_kernel(const T *__restrict__ in, long long n, float scale_max,
+                                                               float *__restrict__ out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = (float)in[i] / scale_max;
+}
+// Arrays that are both 16-byte aligned: `vectors` threads take 16 bytes of
+// texels each, the others the remainder one by one.
+template <typename T>
+__global__ void __launch_bounds__(256) normalize_vectors_kernel(const T *__restrict__ in, long long n, long long vectors,
+                                                                float scale_max, float *__restrict__ out) {
   constexpr int kPer = 16 / sizeof(T);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < vectors) {
@@ -268,11 +275,15 @@ __global__ void __launch_bounds__(256) normalize_texels_kernel(const T *__restri
   if (r < n) out[r] = (float)in[r] / scale_max;
 }
 template <typename T>
-static void launch_normalize(const void *in, long long n, float scale_max, float *out, cudaStream_t stream) {
-  const bool aligned = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
-  const long long per = 16 / sizeof(T), vectors = aligned ? n / per : 0, threads = vectors + (n - vectors * per);
-  normalize_texels_kernel<T><<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(
-      reinterpret_cast<const T *>(in), n, vectors, scale_max, out);
+static gbv_status launch_normalize(const void *in, long long n, float scale_max, float *out, cudaStream_t stream) {
+  const T *t = reinterpret_cast<const T *>(in);
+  if ((((uintptr_t)in | (uintptr_t)out) & 15) != 0) {
+    normalize_texels_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(t, n, scale_max, out);
+    return check_launch("normalize_texels_kernel");
+  }
+  const long long per = 16 / sizeof(T), vectors = n / per, threads = vectors + (n - vectors * per);
+  normalize_vectors_kernel<T><<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(t, n, vectors, scale_max, out);
+  return check_launch("normalize_vectors_kernel");
 }
 
 __global__ void sincos_angle_kernel(const float *__restrict__ x, long long n, float *__restrict__ sn,
@@ -389,9 +400,8 @@ gbv_status gbv_normalize_texels(const void *d_texels, int bits, long long n, flo
   if (!d_texels || !d_scalars || n < 0 || (bits != 8 && bits != 16))
     return set_error(GBV_ERROR_INVALID_ARGUMENT, "gbv_normalize_texels: bad argument (bits must be 8 or 16)");
   if (n == 0) return GBV_OK;
-  if (bits == 8) launch_normalize<uint8_t>(d_texels, n, 255.f, d_scalars, (cudaStream_t)stream);
-  else launch_normalize<uint16_t>(d_texels, n, 65535.f, d_scalars, (cudaStream_t)stream);
-  return check_launch("normalize_texels_kernel");
+  return bits == 8 ? launch_normalize<uint8_t>(d_texels, n, 255.f, d_scalars, (cudaStream_t)stream)
+                   : launch_normalize<uint16_t>(d_texels, n, 65535.f, d_scalars, (cudaStream_t)stream);
 }
 
 }  // extern "C"
