@@ -2253,7 +2253,10 @@ constexpr int kBatchLogPasses = 16;
 // one, and rotating a ray by d changes the ratio of two slab distances by
 // sqrt(2) d or more, against a rounding error of 1e-6 in the float slab test.
 // Where that does not hold (a corner behind or beside the camera, finer
-// pixels, values that are not finite) the rectangle is the whole frame.  A
+// pixels, values that are not finite) the rectangle is the whole frame; where
+// every corner lies behind the plane through the camera, by 1e-3 rad or more,
+// no ray of the frame, all of which lead ahead of it, sees the field (256^3,
+// 1080p, 4 passes, env map: 107 us, 364 as a frame of inner tiles).  A
 // launch of a rank's share of the tiles has no rectangle: rw = 0, every tile
 // is an inner one.
 inline long long plan_rect(RenderParams &p) {
@@ -2269,18 +2272,24 @@ inline long long plan_rect(RenderParams &p) {
   const double corner2 = dd + .25 * aspect * aspect + .25;
   bool whole = !(sqrt(dd) / corner2 / p.H > 1e-5);
   double x0 = 1e30, x1 = -1e30, y0 = 1e30, y1 = -1e30;
-  for (int k = 0; k < 8 && !whole; k++) {
+  bool behind = !whole;  // every corner lies behind the camera
+  for (int k = 0; k < 8; k++) {
     const D3 d{(double)(k & 1 ? p.F.boundsHi.x : p.F.boundsLo.x) - p.lens00.x,
                (double)(k & 2 ? p.F.boundsHi.y : p.F.boundsLo.y) - p.lens00.y,
                (double)(k & 4 ? p.F.boundsHi.z : p.F.boundsLo.z) - p.lens00.z};
     const double t = dotd(d, p.dir00) / dd, len = sqrt(d.x * d.x + d.y * d.y + d.z * d.z);
-    whole = !(t * sqrt(dd) > 1e-3 * len);
+    whole = whole || !(t * sqrt(dd) > 1e-3 * len);
+    behind = behind && t * sqrt(dd) < -1e-3 * len;
     const double x = (.5 + dotd(d, p.du) / t / aspect) * p.W, y = (.5 + dotd(d, p.dv) / t) * p.H;
     whole = whole || !(fabs(x) < 1e9 && fabs(y) < 1e9);
     x0 = x < x0 ? x : x0;
     x1 = x > x1 ? x : x1;
     y0 = y < y0 ? y : y0;
     y1 = y > y1 ? y : y1;
+  }
+  if (behind) {  // nothing of the field is seen: one inner tile, so that rw > 0
+    p.rw = p.rh = 1;
+    return 1;
   }
   if (whole) {
     p.rw = (int)tx;

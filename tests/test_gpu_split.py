@@ -237,3 +237,19 @@ def test_warps_that_give_up_are_reported(cuda, kind, counted):
             assert (counters[N.GBV_COUNTER_CAPS].item() > 0) == (polls == 0)
         if polls:
             np.testing.assert_array_equal(bits(acc.cpu().numpy()), bits(ref.cpu().numpy()))
+
+
+@pytest.mark.parametrize("turn", [60.0, 89.0, 95.0, 135.0, 180.0])
+@pytest.mark.parametrize("fovy", [60.0, 170.0])
+def test_field_beside_and_behind_the_camera(cuda, turn, fovy):
+    """The camera turned away from the field, which is then partly or wholly
+    behind it: the frame is the oracle's."""
+    import torch
+    s = world("dark", 41, 23)
+    s.fovy = fovy
+    d, a = np.array(s.cam_dir, float), np.radians(turn)
+    side = np.cross(d, s.cam_up)
+    s.cam_dir = tuple(np.cos(a) * d + np.sin(a) * side * np.linalg.norm(d) / np.linalg.norm(side))
+    acc = GpuScene(s).render(spp=3)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(bits(acc.cpu().numpy()), bits(oracle.Oracle(s).render(spp=3)))
