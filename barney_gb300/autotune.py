@@ -1,8 +1,9 @@
 """Autotuner for the batched persistent render launch.
 
 The batched launch has knobs that change its speed but never its images
-(every pixel still accumulates in the reference's order, and every brick shape stores the same cells; tests/test_gpu_batch.py
-and tests/test_gpu_bricks.py check both bit for bit):
+(every pixel still accumulates in the reference's order, and every brick shape
+stores the same cells; tests/test_gpu_batch.py and tests/test_gpu_bricks.py
+check both bit for bit):
 
 * brick         -- log2 of the brick edge in cells per axis of the voxel
   stores (where neighbouring cells sit in HBM);

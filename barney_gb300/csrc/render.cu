@@ -206,7 +206,6 @@ static bool resolve_config(const gbv_render_config *c, RenderParams &p, LaunchCh
   if (c->blocks_per_sm) lc.occ = c->blocks_per_sm;
   lc.stage = c->stage;
   if (c->threshold_pct) p.threshold = c->threshold_pct;
-  else if (c->mode == GBV_RENDER_WAVEFRONT) p.threshold = 25;
   if (c->skip_cells) p.skip = lc.skip = c->skip_cells;
   p.profile = c->profile;
   return true;
@@ -352,16 +351,15 @@ extern "C" gbv_status gbv_tile_partition(int width, int height, int rank, int nu
 // real-time viewer that forbids allocation and free calls on its frame
 // path (gbv_render takes its scratch, a long frame's up to 512 MB, from the
 // library's memory pool and keeps it there).  This entry point takes its
-// scratch, two words, from a file-scope device array
-// instead.
+// scratch, two words, from a file-scope device array instead.
 // ===========================================================================
 namespace gbv {
 
 // The only scratch: the tile counters of the frame kernel and of the kernel
-// that finishes the frame (two 32-bit words).  Every GPU that loads this library holds this array until the
-// process exits.  All calls share it and it keeps the last call's value, so
-// each call clears it first; calls that overlap on the GPU (for example on
-// two streams) race on it.
+// that finishes the frame (two 32-bit words).  Every GPU that loads this
+// library holds this array until the process exits.  All calls share it and it
+// keeps the last call's values, so each call clears it first; calls that
+// overlap on the GPU (for example on two streams) race on it.
 static __device__ __align__(256) int g_noalloc_tile_pool[2];
 constexpr long long kNoAllocMaxTiles = 1ll << 30;
 
@@ -388,8 +386,8 @@ extern "C" gbv_status gbv_render_noalloc(const gbv_scene *s, float *d_accum, int
                                          void *stream) {
   if (!s || !d_accum || width <= 0 || height <= 0 || spp < 0 || accum_id_start < 0)
     return set_error(GBV_ERROR_INVALID_ARGUMENT, "gbv_render_noalloc: null pointer or non-positive size");
-  // the scratch is one 32-bit counter of 8x4-pixel tiles; every warp may take
-  // one tile past the end, so the frame's tiles must leave room for them
+  // the scratch is two 32-bit counters of 8x4-pixel tiles; every warp may take
+  // tiles past the end, so the frame's tiles must leave room for them
   const long long tiles = (((long long)width + 7) / 8) * (((long long)height + 3) / 4);
   if (tiles > kNoAllocMaxTiles)
     return set_error(GBV_ERROR_INVALID_ARGUMENT,

@@ -847,21 +847,21 @@ __device__ __forceinline__ void accum_add(float4 &acc, vec3 frag) {
 // position, then the warp's ready lanes take their density samples together.
 // -------------------------------------------------------------------------
 // Defaults of the launch shape and the scheduling limits of the frame kernel
-// (512^3 1080p 16-pass frame / 256^3 720p 1 pass; results never depend on
+// (512^3 1080p 16-pass frame / 256^3 720p 1 pass, ms; results never depend on
 // them):
-// * rounds a seek makes before the warp samples: 2: 12.3 / 0.507 ms, 3:
-//   12.1 / 0.498, 4: 11.7 / 0.502;
+// * rounds a seek makes before the warp samples: 2: 6.59 / 0.508, 3: 6.28 /
+//   0.485, 4: 6.16 / 0.491, 6: 6.16 / 0.505;
 // * a warp leaves tracing for a waiting stage below this share of its lanes:
-//   10%: 12.8 / 0.69, 20%: 12.0 / 0.69, 30%: 11.5 / 0.71, 50%: 11.9 / 0.73,
-//   65%: slower by 10% or more on the small frames;
-// * kRefillMin, the rays a refill waits for: 4: 12.0 / 0.70, 8: 11.8 / 0.69,
-//   12: 11.7 / 0.67;
-// * kFull, the paths that make a stage worth leaving another for: 16: 11.9 /
-//   0.71, 24: 11.8 / 0.69, 30: 11.7 / 0.69.
+//   10%: 6.24 / 0.491, 25%: 6.15 / 0.496, 30%: 6.22 / 0.507, 50%: 7.53 / 0.540,
+//   65%: 11.2 / 0.618;
+// * kRefillMin, the rays a refill waits for: 4: 6.21 / 0.503, 8: 6.11 / 0.493,
+//   12: 6.16 / 0.490;
+// * kFull, the paths that make a stage worth leaving another for: 16: 6.24 /
+//   0.513, 24: 6.18 / 0.496, 28: 6.16 / 0.490, 30: 6.15 / 0.495.
 constexpr int kSkipDefault = 4;
 // A batch's lanes read their scene's record from memory at every seek: one
 // that goes on to its next position reads it less often (64 uneven scenes, 8
-// passes: 4 rounds 6.25 ms, 16: 5.83, 64: 5.53).
+// passes, when this was chosen: 4 rounds 6.25 ms, 16: 5.83, 64: 5.53).
 constexpr int kBatchSkipDefault = 64;
 constexpr int kThresholdDefault = 25;
 constexpr int kRefillMin = 12, kFull = 28;
@@ -1269,8 +1269,10 @@ static __device__ __noinline__ void write_aux(const RenderParams &p, size_t px, 
 // lanes; letting the block's warps leave tracing for shading together
 // (PathPool::shading) keeps them in the same code: 16.2 -> 14.5 ms from the
 // pool, -> 12.4 ms from the common phase, -> 11.7 ms from refilling lanes in
-// batches (512^3, 1080p, 16 passes).  128 registers a thread (16 warps) with
-// next to no spills beat 24 warps of 80 registers (12.9 ms).
+// batches (512^3, 1080p, 16 passes, as each was made; with passes logged, see
+// below, and later changes such a frame takes 6.2 ms).  The register budget
+// matters little to its middle (128 registers a thread 6.27 ms, 96 6.16, 80
+// 6.14) and much to its end, see default_budget.
 //
 // A path that sums all of its pixel's passes runs them one after the other,
 // so the last pixels' passes hold a small frame's end: 50 to 80% of its time.
@@ -2387,7 +2389,7 @@ inline gbv_status plan_grid(RenderParams &p, RenderKernelFn kernel, size_t smemL
 }
 
 // The one-scene render kernels of a launch: with and without event
-// counting, for a volume-only world or (at 4 resident blocks per SM) one
+// counting, for a volume-only world or (with the 128-register budget) one
 // with an iso-surface.
 template <class Store, int Budget>
 inline void render_kernels(const RenderParams &p, RenderKernelFn &counting, RenderKernelFn &plain) {
@@ -2545,8 +2547,8 @@ inline gbv_status launch_render(RenderParams p, const Store &store, cudaStream_t
 
 template <class Store>
 inline gbv_status launch_render_noalloc(RenderParams p, const Store &store, cudaStream_t stream, int *pool) {
-  // fixed launch settings (results do not depend on them): 4 resident
-  // blocks per SM, the default traversal settings, no shared-memory staging
+  // fixed launch settings (results do not depend on them): the 128-register
+  // budget, the default traversal settings, no shared-memory staging
   p.skip = kSkipDefault;
   p.threshold = kThresholdDefault;
   p.idlePolls = kIdlePolls;

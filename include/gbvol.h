@@ -287,10 +287,10 @@ typedef struct gbv_scene {
    [0] density samples, [1] macrocells entered with a non-zero majorant,
    [2] rays traced, [3] loop-cap events, [4] macrocells crossed (all),
    [5..7] SM cycles spent starting passes and shading misses, traversing, and
-   shading hits (with an iso-surface's search), summed over warps, [8] traversal iterations of warps and [9] tracing lanes
-   summed over them, [10] shading passes of warps and [11] shaded lanes
-   summed over them ([5..11] only when gbv_render_ex's config asks for a
-   profile, else 0). */
+   shading hits (with an iso-surface's search), summed over warps,
+   [8] traversal iterations of warps and [9] tracing lanes summed over them,
+   [10] shading passes of warps and [11] shaded lanes summed over them
+   ([5..11] only when gbv_render_ex's config asks for a profile, else 0). */
 enum { GBV_COUNTER_SAMPLES = 0, GBV_COUNTER_MC_VISITS = 1, GBV_COUNTER_RAYS = 2,
        GBV_COUNTER_CAPS = 3, GBV_COUNTER_CELLS = 4, GBV_COUNTER_CYCLES_START = 5,
        GBV_COUNTER_CYCLES_TRAVERSE = 6, GBV_COUNTER_CYCLES_SHADE = 7,
